@@ -89,15 +89,23 @@ static __constant__ u32 g_pow2[32] = {1u, 2u, 4u, 8u, 16u, 32u, 64u, 128u, 256u,
                                       536870912u, 1073741824u, 2147483648u};
 __device__ __forceinline__ u32 fmul32(u32 a, u32 m)
 {
+#ifdef __CUDACC__
     u32 d;
     asm("mul.lo.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(m));
     return d;
+#else  // host compilation of these headers
+    return a * m;
+#endif
 }
 __device__ __forceinline__ u32 fmad32(u32 a, u32 m, u32 c)
 {
+#ifdef __CUDACC__
     u32 d;
     asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(m), "r"(c));
     return d;
+#else
+    return a * m + c;
+#endif
 }
 // x << K (0 < K < 64)
 template <int K> __device__ __forceinline__ u64 shl(u64 x)

@@ -13,15 +13,17 @@
 //                   a shared queue and writes children coalesced in 16-byte
 //                   vectors (replaces IntervalExpand + generate_moves +
 //                   makemove_and_count, perft_bb.h:601,983; intervalmove.cuh:405)
-//   k_leaf          the last two plies inside one CTA: count each node's
-//                   moves, scan in shared memory, queue (parent, move)
-//                   entries, then every thread makes + counts entries, so
-//                   the per-thread work is even whatever the branching
+//   k_leaf          the last two plies inside one CTA: each thread sums one
+//                   node's replies to its plain moves in sets (pg_reply.cuh)
+//                   and queues the other moves as (parent, move) entries, then
+//                   every thread makes + counts entries, so the per-thread
+//                   work is even whatever the branching
 //                   (replaces makeMove_and_perft_single_level_indices,
 //                   perft_bb.h:412)
 #pragma once
 #include "pg_level.cuh"
 #include "pg_movegen.cuh"
+#include "pg_reply.cuh"
 
 namespace pg {
 
@@ -88,11 +90,6 @@ __device__ __forceinline__ u32 block_excl_scan(u32 v, u32& total, u32* s_warp)
 struct QEmit {
     u32* q;
     u32 pos, lo, hi, tag;
-    __device__ __forceinline__ void operator()(u16 m)
-    {
-        if (pos >= lo && pos < hi) q[pos - lo] = tag | m;
-        ++pos;
-    }
     // bits 25-28 carry the moving piece (PC_*) and PC_EP_FLAG for make_child
     __device__ __forceinline__ void operator()(u16 m, u32 piece)
     {
@@ -101,13 +98,46 @@ struct QEmit {
     }
 };
 
-// QEmit when every move of the CTA's nodes fits the queue (one window)
-struct QEmitAll {
+// reply_sum's emitter for the leaf: entries are reserved from the CTA's
+// counter, and dropped (only counted) beyond the queue's end; the landing
+// piece goes to bits 25-28 as in QEmit
+template <int QCAP> struct QTake {
     u32* q;
-    u32 pos, tag;
-    __device__ __forceinline__ void operator()(u16 m) { q[pos++] = tag | m; }
-    __device__ __forceinline__ void operator()(u16 m, u32 piece) { q[pos++] = tag | m | (piece << 25); }
+    u32* queued;
+    u32 tag, taken;
+    __device__ __forceinline__ u32 take(u32 k)
+    {
+        taken += k;
+        return atomicAdd(queued, k);
+    }
+    __device__ __forceinline__ void put(u32 at, u16 m, u32 piece)
+    {
+        if (at < (u32)QCAP) q[at] = tag | m | (piece << 25);
+    }
 };
+
+// the same moves again at fixed positions: those in [lo, hi) are written
+struct QWindow {
+    u32* q;
+    u32 pos, lo, hi, tag;
+    __device__ __forceinline__ u32 take(u32 k)
+    {
+        const u32 at = pos;
+        pos += k;
+        return at;
+    }
+    __device__ __forceinline__ void put(u32 at, u16 m, u32 piece)
+    {
+        if (at >= lo && at < hi) q[at - lo] = tag | m | (piece << 25);
+    }
+};
+// one node's part of a queue window (rare: a CTA with more children than its
+// queue holds), out of line so that the leaf keeps one copy of reply_sum
+template <int S> __device__ __noinline__ void queue_window(const Pos& b, u32* q, u32 off, u32 lo, u32 hi, u32 tag)
+{
+    QWindow e{q, off, lo, hi, tag};
+    reply_sum<S>(b, ks_facts<S>(b), e);
+}
 
 struct ArrEmit {
     u16* out;

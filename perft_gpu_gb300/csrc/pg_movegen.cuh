@@ -46,6 +46,7 @@ static __device__ u64 g_knight_t[65];
 static __device__ u64 g_king[64];
 static __device__ u64 g_diag[64];
 static __device__ u64 g_pawn_checks[2][64];
+static __device__ u64 g_between[64][64];  // squares strictly between two squares of one line
 // The count is bound by integer-ALU issue (the ALU pipe ~88-91% busy, the
 // FMA pipe ~10-14%).  Its popcount sums are written as multiply-adds by a 1 the
 // compiler cannot fold (a __constant__ word), so they issue on the FMA pipe
@@ -54,9 +55,7 @@ static __device__ u64 g_pawn_checks[2][64];
 static __constant__ u32 g_fma_one = 1;
 __device__ __forceinline__ u32 fma_add(u32 a, u32 b)
 {
-    u32 d;
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(g_fma_one), "r"(b));
-    return d;
+    return fmad32(a, g_fma_one, b);
 }
 // o - 2m per 32-bit half, as multiply-adds by -2 on the FMA pipe; equal to
 // the 64-bit o - 2m when no borrow leaves bit 31 (bit 31 of o set).  The rank
@@ -65,9 +64,7 @@ __device__ __forceinline__ u32 fma_add(u32 a, u32 b)
 static __constant__ u32 g_fma_m2 = 0xFFFFFFFEu;
 __device__ __forceinline__ u64 sub2_halves(u64 o, u64 m)
 {
-    u32 lo, hi;
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(lo) : "r"((u32)m), "r"(g_fma_m2), "r"((u32)o));
-    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(hi) : "r"((u32)(m >> 32)), "r"(g_fma_m2), "r"((u32)(o >> 32)));
+    const u32 lo = fmad32((u32)m, g_fma_m2, (u32)o), hi = fmad32((u32)(m >> 32), g_fma_m2, (u32)(o >> 32));
     return ((u64)hi << 32) | lo;
 }
 // n + popcount(x), the additions on the FMA pipe
@@ -85,6 +82,7 @@ static inline cudaError_t upload_static_tables(const HostTables& t)
     if ((e = cudaMemcpyToSymbol(g_king, t.king, sizeof(t.king)))) return e;
     if ((e = cudaMemcpyToSymbol(g_diag, t.diag, sizeof(t.diag)))) return e;
     if ((e = cudaMemcpyToSymbol(g_pawn_checks, t.pawn_checks, sizeof(t.pawn_checks)))) return e;
+    if ((e = cudaMemcpyToSymbol(g_between, t.between, sizeof(t.between)))) return e;
     if ((e = cudaMemcpyToSymbol(g_knight, t.knight, sizeof(t.knight)))) return e;
     {
         u64 kt[65];
@@ -455,7 +453,9 @@ __device__ __forceinline__ u32 count_from_facts(const Pos& b, const KsFacts<S>& 
         // opaque copy of `empty`, so the compiler builds them here rather than
         // early, where they would be live across pass 1.
         u64 empty2 = empty;
+#ifdef __CUDACC__
         asm volatile("" : "+l"(empty2));
+#endif
         {
             const u64 ns = my_rq & ~((pinned ^ pf) | pin_chk);
             u64 up_att, down_att;
@@ -807,6 +807,30 @@ template <class E> __device__ __forceinline__ void emit_pawn_sq(E& emit, int fro
     }
 }
 
+// castles and en-passant captures
+template <int S, class E> __device__ __forceinline__ void emit_castles_ep(const Pos& b, const KsFacts<S>& f, E&& emit)
+{
+    if (!f.checkers) {
+        if (can_castle_k<S>(b, f.occ, f.threat)) emit(cmove(S ? 60 : 4, S ? 62 : 6, MF_KCASTLE), PC_KING);
+        if (can_castle_q<S>(b, f.occ, f.threat)) emit(cmove(S ? 60 : 4, S ? 58 : 2, MF_QCASTLE), PC_KING);
+    }
+    // en passant: the rules of count_ep_ks
+    if (b.p & 0xF0ull) {
+        const u64 et = ep_target<S>(b);
+        const u64 victim = S ? up(et) : down(et);
+        const int to = lsb(et) & 63;
+        u64 cand = (east1(victim) | west1(victim)) & f.pawns & f.mine;
+        if (f.checkers) {
+            cand = (victim == f.checkers) ? (cand & ~f.pinned) : 0ull;
+            for (; cand; cand &= cand - 1) emit(cmove(lsb(cand), to, MF_EP), PC_PAWN);
+        } else {
+            const Sides<S> c(b);
+            for (; cand; cand &= cand - 1)
+                if (ep_legal<S>(c, f.pinned, lowbit(cand), et, victim)) emit(cmove(lsb(cand), to, MF_EP), PC_PAWN);
+        }
+    }
+}
+
 template <int S, class E> __device__ __forceinline__ void gen_from_facts(const Pos& b, const KsFacts<S>& f, E& emit)
 {
     const u64 tgt = f.tgt;
@@ -852,25 +876,7 @@ template <int S, class E> __device__ __forceinline__ void gen_from_facts(const P
                 [&](int to) { emit_pawn_sq(emit, to - CW, to, 0); });
     each_square(cap_e<S>(fp | (myp & (S ? f.pa : f.pd) & pin_ok)) & f.theirs & tgt,
                 [&](int to) { emit_pawn_sq(emit, to - CE, to, 0); });
-    if (!f.checkers) {
-        if (can_castle_k<S>(b, f.occ, f.threat)) emit(cmove(S ? 60 : 4, S ? 62 : 6, MF_KCASTLE), PC_KING);
-        if (can_castle_q<S>(b, f.occ, f.threat)) emit(cmove(S ? 60 : 4, S ? 58 : 2, MF_QCASTLE), PC_KING);
-    }
-    // en passant: the rules of count_ep_ks
-    if (b.p & 0xF0ull) {
-        const u64 et = ep_target<S>(b);
-        const u64 victim = S ? up(et) : down(et);
-        const int to = lsb(et) & 63;
-        u64 cand = (east1(victim) | west1(victim)) & myp;
-        if (f.checkers) {
-            cand = (victim == f.checkers) ? (cand & ~f.pinned) : 0ull;
-            for (; cand; cand &= cand - 1) emit(cmove(lsb(cand), to, MF_EP));
-        } else {
-            const Sides<S> c(b);
-            for (; cand; cand &= cand - 1)
-                if (ep_legal<S>(c, f.pinned, lowbit(cand), et, victim)) emit(cmove(lsb(cand), to, MF_EP));
-        }
-    }
+    emit_castles_ep<S>(b, f, emit);
 }
 
 template <int S, class E> __device__ __forceinline__ void gen_leaf(const Pos& b, E& emit)
@@ -1068,10 +1074,14 @@ __device__ __forceinline__ void make_move(Pos& b, u16 mv)
 // 64-bit variable shift)
 __device__ __forceinline__ u64 bit64(u32 s)
 {
+#ifdef __CUDACC__
     u32 lo, hi;
     asm("shl.b32 %0, %1, %2;" : "=r"(lo) : "r"(1u), "r"(s));
     asm("shl.b32 %0, %1, %2;" : "=r"(hi) : "r"(1u), "r"(s - 32u));
     return ((u64)hi << 32) | lo;
+#else
+    return 1ull << s;
+#endif
 }
 
 // makeMove for a child whose moves are only counted: it writes what the count

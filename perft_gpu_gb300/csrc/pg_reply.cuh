@@ -1,0 +1,467 @@
+// pg_reply.cuh -- the last two plies of a position without making most of
+// its moves.
+//
+// perft(2) of a position is the sum, over the legal moves of the side to move
+// (the mover), of the number of replies.  Most moves change few of the
+// replies: the opponent's reply count after such a move is its count on the
+// unmoved board (the mover passes) plus a correction that depends on the
+// square left and the square reached alone.  reply_sum splits the moves:
+//
+//  * plain moves are counted in sets: per moving piece the popcount of its
+//    plain targets times (passed count + correction for the square left), and
+//    over all pieces the corrections for the squares reached, as popcounts of
+//    bit planes (a square's correction in binary, one 64-bit mask per digit);
+//  * every other move (a check, a discovered line, a change of the squares the
+//    king may enter, castling, promotion, en passant, ...) goes to the
+//    emitter, and is made and counted as before.
+//
+// A move from f to t by piece X is plain when, with K the opponent's king:
+//  1. K is not attacked on the unmoved board (else no move is plain);
+//  2. f and t change no pin and no check: f is not a blocker whose leaving
+//     opens a line of another mover's slider to K or pins a piece, nor a
+//     pinner; t is not on a line X itself then looks along to K through at most
+//     one opposing piece; t does not unpin or capture a pinned piece;
+//  3. the squares K may enter (and cross when castling) are attacked or not
+//     as before: X attacks none of the attacked ones from f alone and none of
+//     the free ones from t, no slider's line through f or t reaches one, and
+//     neither f nor t is next to K or on a castling path;
+//  4. f and t do not share a line of an opposing slider that sees f, and t is
+//     not a piece whose own count the square left has already corrected.
+// Then the replies change only by
+//  * the opponent's sliders (pinned ones do not see f or t): the rays that
+//    ended on f run on, the rays that passed t end there;
+//  * its pawns: pushes onto f and t, captures on f and t;
+//  * a captured piece: its own moves go, and the pieces that defend t (sliders,
+//    knights, pawns) gain the recapture.
+// The legality rules enter only through the passed count, whose terms are
+// count_moves_ks1's outside check.
+//
+// What bounds it: integer-ALU issue, as the count of a made child (about 650
+// instructions); the set-wise part costs a node a few children's worth and
+// replaces 71% of its children (batched uneven workload, 34 moves a node).
+// Measured (GB300): 4,096 positions at depths 3..6 in 653 ms against 1,222 ms
+// with every child made and counted; one position at depth 7 in 23.0 against
+// 46.6 ms.
+#pragma once
+#include "pg_movegen.cuh"
+
+namespace pg {
+
+// sum and carry of three bit planes
+__device__ __forceinline__ u64 plane_sum(u64 a, u64 b, u64 c) { return a ^ b ^ c; }
+__device__ __forceinline__ u64 plane_carry(u64 a, u64 b, u64 c) { return (a & b) | (c & (a | b)); }
+
+// a three-digit number per square
+struct Planes3 {
+    u64 c0, c1, c2;
+};
+
+// How many targets an opposing slider's ray still has beyond each square it
+// passes, and beyond the slider itself (its moves along the ray): 0..7 per
+// square.  v: the attack fill of the sliders along one direction (blockers
+// included), own: the sliders' side (not a target), sl: the sliders.  The run
+// of targets is followed back one step at a time, through empty squares only.
+template <int SH, bool LEFT> __device__ __forceinline__ Planes3 targets_beyond(u64 v, u64 empty, u64 own, u64 sl)
+{
+    const u64 through = v & empty, at = through | sl;
+    auto back = [](u64 x) { return LEFT ? (x >> SH) : (x << SH); };
+    const u64 r1 = back(v & ~own) & at;
+    const u64 r2 = back(r1 & through) & at;
+    const u64 r3 = back(r2 & through) & at;
+    const u64 r4 = back(r3 & through) & at;
+    const u64 r5 = back(r4 & through) & at;
+    const u64 r6 = back(r5 & through) & at;
+    const u64 r7 = back(r6 & through) & at;
+    return Planes3{(r1 & ~r2) | (r3 & ~r4) | (r5 & ~r6) | r7, (r2 & ~r4) | r6, r4};
+}
+
+// a pawn move by target square; on rank 1 or 8 the four promotions, as emit_pawn_sq
+template <class E> __device__ __forceinline__ void put_pawn(E& emit, u32& at, int from, int to, int fl)
+{
+    auto one = [&](u16 mv, u32 piece) { emit.put(at++, mv, piece); };
+    emit_pawn_sq(one, from, to, fl);
+}
+
+// The replies to the plain moves of b (S to move; f = ks_facts of b), summed;
+// every other move goes to emit: emit.take(n) reserves n entries and returns
+// the first one's position, emit.put(position, move, landing piece).
+template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b, const KsFacts<S>& f, E& emit)
+{
+    constexpr int T = 1 - S;
+    const u64 mine = f.mine, own = f.theirs, occ = f.occ, empty = f.empty, pawns = f.pawns;
+    const u64 mrq = b.rq & mine, mbq = b.bq & mine, mp = pawns & mine, mn = b.n & mine, mk = b.k & mine;
+    const u64 king = b.k & own;
+    const int kq = sq_of(king);
+    const u64 kr = SlFancy::rook(kq, occ), kb = SlFancy::bishop(kq, occ);
+    const u64 ring = __ldg(&g_king[kq]);
+
+    // squares a plain move may not leave / reach, whatever the piece
+    u64 no_f = ring, no_t = ring;
+    // the opponent's king attacked with the mover to move: nothing is plain
+    if ((kr & mrq) | (kb & mbq) | (__ldg(&g_knight[kq]) & mn) | (__ldg(&g_pawn_checks[T][kq]) & mp) | (ring & mk)) {
+        no_f = ~0ull;
+        no_t = ~0ull;
+    }
+
+    // the mover's sliders on K's lines: the opponent's pins, and the blockers
+    // that may not leave
+    u64 pf = 0, pr = 0, pd = 0, pa = 0;
+    {
+        const u64 lf = file_of(kq), lr = rank_of(kq), ld = __ldg(&g_diag[kq]), la = anti_of(kq);
+        for (u64 s = ((lf | lr) & mrq) | ((ld | la) & mbq); s; s &= s - 1) {
+            const int q = lsb(s);
+            const u64 sb = lowbit(s);
+            const u64 between = __ldg(&g_between[kq][q]);
+            const u64 in = between & occ;
+            const int n = popc(in);
+            if (n == 1) {
+                if (in & own) {
+                    pf |= (lf & sb) ? in : 0ull;
+                    pr |= (lr & sb) ? in : 0ull;
+                    pd |= (ld & sb) ? in : 0ull;
+                    pa |= (la & sb) ? in : 0ull;
+                    no_t |= between;
+                    no_f |= sb;
+                } else {
+                    no_f |= in;
+                }
+            } else if (n == 2) {
+                const u64 m = in & mine;
+                no_f |= (m != in) ? m : 0ull;
+            }
+        }
+    }
+    const u64 pinned = pf | pr | pd | pa;
+
+    const VPro v(empty);
+    const RankPro h(occ);
+    const u64 pass = empty & NOT_A & NOT_H;
+    const DPro<9> d9(pass);
+    const DPro<7> d7(pass);
+
+    // castling squares of the opponent that its own pieces leave open
+    u64 path = 0, cross = 0;
+    if (b.p & (T ? 0xCull : 0x3ull)) {
+        const int rights = T ? st_bc(b) : st_wc(b);
+        constexpr u64 kp = T ? B_KS_PATH : W_KS_PATH, qp = T ? B_QS_PATH : W_QS_PATH, qs = T ? B_QS_SAFE : W_QS_SAFE;
+        if ((rights & 1) && !(kp & own)) { path |= kp; cross |= kp; }
+        if ((rights & 2) && !(qp & own)) { path |= qp; cross |= qs; }
+        no_f |= path;
+        no_t |= path | (path ? (T ? 0x81ull << 56 : 0x81ull) : 0ull);  // a captured corner rook takes the right
+    }
+
+    // the squares K may enter or cross: free (u0) or attacked, and those attacked once
+    u64 u0, u_once, thr, tr, tb;
+    {
+        const u64 a0 = v.up(mrq), a1 = v.down(mrq), a2 = h.east(mrq), a3 = h.west(mrq);
+        const u64 a4 = d9.up(mbq), a5 = d9.down(mbq), a6 = d7.up(mbq), a7 = d7.down(mbq);
+        u64 once = a0, twice = 0;
+        auto add = [&](u64 x) { twice |= once & x; once |= x; };
+        add(a1); add(a2); add(a3); add(a4); add(a5); add(a6); add(a7);
+        add(cap_w<S>(mp));
+        add(cap_e<S>(mp));
+        for (u64 s = mn; s; s &= s - 1) add(__ldg(&g_knight[lsb(s)]));
+        add(__ldg(&g_king[sq_of(mk)]));
+        thr = once;
+        const u64 u = (ring & ~own) | cross;
+        u0 = u & ~thr;
+        const u64 u1 = u & thr;
+        u_once = u1 & ~twice;
+        // from where a slider reaches them: fills backward from the squares
+        // (on ranks through a board where they are blockers, as the rank fill
+        // needs its sources occupied); a slider's own fill along the same
+        // direction meets them on the lines that a blocker leaving (free
+        // squares) or a piece arriving (attacked ones) changes
+        {
+            const RankPro g(occ | u0);
+            const u64 b0 = v.down(u0), b1 = v.up(u0), b2 = g.west(u0), b3 = g.east(u0);
+            const u64 b4 = d9.down(u0), b5 = d9.up(u0), b6 = d7.down(u0), b7 = d7.up(u0);
+            tr = b0 | b1 | b2 | b3;
+            tb = b4 | b5 | b6 | b7;
+            no_f |= (a0 & b0) | (a1 & b1) | (a2 & b2) | (a3 & b3) | (a4 & b4) | (a5 & b5) | (a6 & b6) | (a7 & b7);
+        }
+        {
+            const RankPro g(occ | u1);
+            no_t |= ((a0 & v.down(u1)) | (a1 & v.up(u1)) | (a2 & g.west(u1)) | (a3 & g.east(u1)) | (a4 & d9.down(u1)) |
+                     (a5 & d9.up(u1)) | (a6 & d7.down(u1)) | (a7 & d7.up(u1))) & empty;
+        }
+        // a slider arriving on K's lines checks, or pins the one piece between
+        tr |= SlFancy::rook(kq, occ ^ (kr & own));
+        tb |= SlFancy::bishop(kq, occ ^ (kb & own));
+    }
+    const u64 tn = knight_set(u0 | king), tk = king_set(u0);
+
+    // ---- the opponent's moves on the unmoved board ----
+    const u64 free_ = own & ~pinned;
+    const u64 orq = b.rq & free_, obq = b.bq & free_, op = pawns & free_;
+    u32 n0 = popc(u0 & ring);
+    for (u64 s = pinned & (b.rq | b.bq); s; s &= s - 1) {
+        const int q = lsb(s);
+        const u64 bit = lowbit(s);
+        u64 m = (b.rq & bit) ? SlFancy::rook(q, occ) : 0ull;
+        if (b.bq & bit) m |= SlFancy::bishop(q, occ);
+        n0 += popc(m & ~own & ((pf & bit) ? file_of(kq) : (pr & bit) ? rank_of(kq) : (pd & bit) ? __ldg(&g_diag[kq]) : anti_of(kq)));
+    }
+    constexpr u64 back_rank = T ? RANK_1 : RANK_8, last_rank = T ? RANK_1 << 8 : RANK_8 >> 8;
+    const u64 d1 = push1<T>(op) & empty;
+    const u64 mid = d1 & double_rank<T>();
+    const u64 dd = push1<T>(mid) & empty;
+    const u64 cw = cap_w<T>(op), ce = cap_e<T>(op);
+    {
+        const u64 opn = pawns & own;
+        const u64 x1 = push1<T>(op | (opn & pf)) & empty;
+        n0 += popc(x1) + popc(push1<T>(x1 & double_rank<T>()) & empty);
+        const u64 xw = cap_w<T>(op | (opn & (T ? pd : pa))) & mine;
+        const u64 xe = cap_e<T>(op | (opn & (T ? pa : pd))) & mine;
+        n0 += popc(xw) + popc(xe);
+        n0 += 3 * (popc(x1 & back_rank) + popc(xw & back_rank) + popc(xe & back_rank));
+        if (path) n0 += can_castle_k<T>(b, occ, thr) + can_castle_q<T>(b, occ, thr);
+    }
+    // promotion squares count four times: not plain; neither is a piece that
+    // blocks a double push
+    const u64 fronts = push1<T>(op) & mine;
+    {
+        const u64 pr8 = (push1<T>(op) | cw | ce) & back_rank;
+        no_t |= pr8;
+        no_f |= pr8 | (fronts & double_rank<T>()) | push1<T>(mid);
+    }
+
+    // w: per square the replies lost when a piece arrives, plus 2: on an empty
+    // square the rays cut off, the pushes blocked and (as 1 - x) the pawn
+    // captures gained; on an opposing piece its moves and (as 1 - x) the pawn
+    // recaptures gained.  g: the sliders and knights that recapture.
+    u64 w0, w1, w2, w3, g0, g1, g2;
+    {
+        const u64 s0 = v.up(orq), s1 = v.down(orq), s2 = h.east(orq), s3 = h.west(orq);
+        const u64 s4 = d9.up(obq), s5 = d9.down(obq), s6 = d7.up(obq), s7 = d7.down(obq);
+        n0 += popc(s0 & ~own) + popc(s1 & ~own) + popc(s2 & ~own) + popc(s3 & ~own) + popc(s4 & ~own) + popc(s5 & ~own) +
+              popc(s6 & ~own) + popc(s7 & ~own);
+        // knights: their moves at their squares, and the first two's attacks
+        u64 kc0 = 0, kc1 = 0, kc2 = 0, kc3 = 0, k1 = 0, k2 = 0;
+        for (u64 s = b.n & free_; s; s &= s - 1) {
+            const u64 bit = lowbit(s), m = __ldg(&g_knight[lsb(s)]);
+            const u32 c = popc(m & ~own);
+            n0 += c;
+            const u32 c7 = c - (c >> 3);  // 8 as 7 + 1
+            kc0 |= (c7 & 1) ? bit : 0ull;
+            kc1 |= (c7 & 2) ? bit : 0ull;
+            kc2 |= (c7 & 4) ? bit : 0ull;
+            kc3 |= (c & 8) ? bit : 0ull;
+            no_t |= k2 & m & own;  // three knights recapture: not plain
+            k2 |= k1 & m;
+            k1 |= m;
+        }
+        // k1: attacked by a knight, k2: by two or more
+        {
+            const u64 x0 = plane_sum(s0, s1, s2), y0 = plane_carry(s0, s1, s2);
+            const u64 x1 = plane_sum(s3, s4, s5), y1 = plane_carry(s3, s4, s5);
+            const u64 kk = k1 & ~k2;
+            const u64 x2 = plane_sum(s6, s7, kk), y2 = plane_carry(s6, s7, kk);
+            g0 = plane_sum(x0, x1, x2);
+            const u64 y3 = plane_carry(x0, x1, x2);
+            const u64 z0 = plane_sum(y0, y1, y2), c0 = plane_carry(y0, y1, y2);
+            g1 = plane_sum(z0, y3, k2);
+            const u64 c1 = plane_carry(z0, y3, k2);
+            g2 = c0 ^ c1;
+            no_t |= c0 & c1 & own;  // eight or more: not plain
+            g0 &= own;
+            g1 &= own;
+            g2 &= own;
+        }
+        Planes3 q0 = targets_beyond<8, true>(s0, empty, own, orq), q1 = targets_beyond<8, false>(s1, empty, own, orq);
+        Planes3 q2 = targets_beyond<1, true>(s2, empty, own, orq), q3 = targets_beyond<1, false>(s3, empty, own, orq);
+        Planes3 q4 = targets_beyond<9, true>(s4, empty, own, obq), q5 = targets_beyond<9, false>(s5, empty, own, obq);
+        const Planes3 q6 = targets_beyond<7, true>(s6, empty, own, obq), q7 = targets_beyond<7, false>(s7, empty, own, obq);
+        // knights' and pawns' moves at their own squares, where the slider
+        // planes are zero
+        q0.c0 |= kc0;
+        q0.c1 |= kc1;
+        q0.c2 |= kc2;
+        q2.c0 |= kc3;
+        {
+            const u64 m1 = push1<S>(d1), m2 = push1<S>(push1<S>(dd));
+            const u64 mw = T ? (cw & mine) << 9 : (cw & mine) >> 7, me = T ? (ce & mine) << 7 : (ce & mine) >> 9;
+            q0.c0 |= m1 & ~last_rank;
+            q0.c2 |= m1 & last_rank;
+            q1.c0 |= m2;
+            q2.c0 |= mw & ~last_rank;
+            q2.c2 |= mw & last_rank;
+            q4.c0 |= me & ~last_rank;
+            q4.c2 |= me & last_rank;
+        }
+        // per line at most 7 (on an empty square at most 6, so the push planes
+        // fit as carries), then the four lines and the capture planes
+        u64 c;
+        const u64 pd2 = dd | push1<S>(dd);
+        const u64 f0 = plane_sum(q0.c0, q1.c0, d1);
+        c = plane_carry(q0.c0, q1.c0, d1);
+        const u64 f1 = plane_sum(q0.c1, q1.c1, c), f2 = q0.c2 ^ q1.c2 ^ plane_carry(q0.c1, q1.c1, c);
+        const u64 r0 = plane_sum(q2.c0, q3.c0, pd2);
+        c = plane_carry(q2.c0, q3.c0, pd2);
+        const u64 r1 = plane_sum(q2.c1, q3.c1, c), r2 = q2.c2 ^ q3.c2 ^ plane_carry(q2.c1, q3.c1, c);
+        const u64 e0 = q4.c0 ^ q5.c0;
+        c = q4.c0 & q5.c0;
+        const u64 e1 = plane_sum(q4.c1, q5.c1, c), e2 = q4.c2 ^ q5.c2 ^ plane_carry(q4.c1, q5.c1, c);
+        const u64 i0 = q6.c0 ^ q7.c0;
+        c = q6.c0 & q7.c0;
+        const u64 i1 = plane_sum(q6.c1, q7.c1, c), i2 = q6.c2 ^ q7.c2 ^ plane_carry(q6.c1, q7.c1, c);
+        const u64 a0 = plane_sum(f0, r0, ~cw);
+        c = plane_carry(f0, r0, ~cw);
+        const u64 a1 = plane_sum(f1, r1, c);
+        c = plane_carry(f1, r1, c);
+        const u64 a2 = plane_sum(f2, r2, c), a3 = plane_carry(f2, r2, c);
+        const u64 b0 = plane_sum(e0, i0, ~ce);
+        c = plane_carry(e0, i0, ~ce);
+        const u64 b1 = plane_sum(e1, i1, c);
+        c = plane_carry(e1, i1, c);
+        const u64 b2 = plane_sum(e2, i2, c), b3 = plane_carry(e2, i2, c);
+        w0 = a0 ^ b0;
+        c = a0 & b0;
+        w1 = plane_sum(a1, b1, c);
+        c = plane_carry(a1, b1, c);
+        w2 = plane_sum(a2, b2, c);
+        c = plane_carry(a2, b2, c);
+        w3 = plane_sum(a3, b3, c);
+        no_t |= plane_carry(a3, b3, c);  // 16 or more: not plain
+    }
+    n0 += 2;
+
+    // ---- the mover's moves ----
+    // m: how many plain moves reach each square (0..7; a square already
+    // reached by seven is not plain for the next piece)
+    u64 m0 = 0, m1 = 0, m2 = 0;
+    u32 sum = 0;
+    auto reach = [&](u64 s) {
+        const u64 k0 = m0 & s;
+        m0 ^= s;
+        const u64 k1 = m1 & k0;
+        m1 ^= k0;
+        m2 ^= k1;
+    };
+    auto full = [&]() { return m0 & m1 & m2; };
+
+    const u64 tgt = f.tgt;
+    const int ksq = f.ksq;
+    const u64 pin_chk = f.pinned & f.chk_all;
+    for (u64 s = mk | (mn & ~f.pinned) | ((mrq | mbq) & ~pin_chk); s; s &= s - 1) {
+        const int q = lsb(s);
+        const u64 bit = lowbit(s);
+        const bool is_k = (mk & bit) != 0, is_n = (mn & bit) != 0, is_r = (mrq & bit) != 0, is_b = (mbq & bit) != 0;
+        const u64 ra = SlFancy::rook(q, occ), ba = SlFancy::bishop(q, occ);
+        const u64 att = is_k ? __ldg(&g_king[q]) : is_n ? __ldg(&g_knight[q]) : ((is_r ? ra : 0ull) | (is_b ? ba : 0ull));
+        u64 to = att & (is_k ? ~(f.threat | mine) : tgt);
+        if (f.pinned & bit)
+            to &= (f.pf & bit) ? file_of(ksq) : (f.pr & bit) ? rank_of(ksq) : (f.pd & bit) ? __ldg(&g_diag[ksq]) : anti_of(ksq);
+        // the square left: pawns that could capture or were blocked there, and
+        // the opposing sliders' rays that run on (t on such a line: not plain)
+        u64 no = no_t | full() | (is_k ? tk : is_n ? tn : ((is_r ? tr : 0ull) | (is_b ? tb : 0ull)));
+        const u64 pawn_att = __ldg(&g_pawn_checks[S][q]) & op;
+        const u64 front = push1<S>(fronts & bit);
+        no |= pawn_att | front;
+        u32 gain = n0 + (front != 0) - popc(pawn_att);
+        for (u64 x = (ra & orq) | (ba & obq); x; x &= x - 1) {
+            const int a = lsb(x);
+            const u64 ab = lowbit(x);
+            const u64 fl = file_of(q), dg = __ldg(&g_diag[q]);
+            const u64 line = (ra & ab) ? ((fl & ab) ? ra & fl : ra & ~fl) : ((dg & ab) ? ba & dg : ba & ~dg);
+            no |= line;
+            gain += popc(line & ~own & (a < q ? ~(bit | (bit - 1)) : bit - 1));
+        }
+        if ((bit & no_f) | (att & u_once)) no = ~0ull;
+        const u64 plain = to & ~no;
+        reach(plain);
+        sum += popc(plain) * gain;
+        const u64 rest = to & no;
+        if (rest) {
+            u32 at = emit.take(popc(rest));
+            const u32 pc = is_k ? PC_KING : is_n ? PC_KNIGHT : is_r ? (is_b ? PC_QUEEN : PC_ROOK) : PC_BISHOP;
+            each_square(rest, [&](int t) { emit.put(at++, cmove(q, t, 0), pc); });
+        }
+    }
+
+    // pawns, by target square; from = to - step
+    constexpr int PUSH = S ? -8 : 8, CW = S ? -9 : 7, CE = S ? -7 : 9;
+    const u64 fp = mp & ~f.pinned;
+    const u64 pin_ok = ~f.chk_all;
+    const u64 x1 = push1<S>(fp | (mp & f.pf & pin_ok)) & empty;
+    const u64 one = x1 & tgt;
+    const u64 two = push1<S>(x1 & double_rank<S>() & ~f.safe) & empty & tgt;
+    const u64 xw = cap_w<S>(fp | (mp & (S ? f.pd : f.pa) & pin_ok)) & own & tgt;
+    const u64 xe = cap_e<S>(fp | (mp & (S ? f.pa : f.pd) & pin_ok)) & own & tgt;
+    {
+        // squares a pawn may not leave, those where an opposing slider's ray
+        // that runs on (pushes: not along the file) is not corrected for, and
+        // squares it may not reach
+        const u64 stay = no_f | cap_w<T>(u_once) | cap_e<T>(u_once) | fronts;
+        const u64 sv0 = v.up(orq) | v.down(orq);
+        const u64 so2 = h.east(orq), so3 = h.west(orq), so4 = d9.up(obq), so5 = d9.down(obq), so6 = d7.up(obq), so7 = d7.down(obq);
+        const u64 seen = sv0 | so2 | so3 | so4 | so5 | so6 | so7;
+        const u64 no = no_t | pawn_attackers_of<T>(u0 | king) | BACK_RANKS;
+        {
+            const u64 ok = one & ~(no | full()) & ~push1<S>(stay | sv0);
+            const u64 from = push1<T>(ok);
+            reach(ok);
+            const u64 nown = ~own;
+            sum += popc(ok) * n0 - popc(from & cw) - popc(from & ce) + popc(h.east(so2 & from) & nown) +
+                   popc(h.west(so3 & from) & nown) + popc(d9.up(so4 & from) & nown) + popc(d9.down(so5 & from) & nown) +
+                   popc(d7.up(so6 & from) & nown) + popc(d7.down(so7 & from) & nown);
+            const u64 rest = one & ~ok;
+            if (rest) {
+                u32 at = emit.take(popc(rest) + 3 * popc(rest & BACK_RANKS));
+                each_square(rest, [&](int t) { put_pawn(emit, at, t - PUSH, t, 0); });
+            }
+        }
+        {
+            const u64 ep = (pawns & own);
+            const u64 epf = two & (east1(ep) | west1(ep));
+            const u64 ok = two & ~(no | full() | epf) & ~push1<S>(push1<S>(stay | seen));
+            const u64 from = push1<T>(push1<T>(ok));
+            reach(ok);
+            sum += popc(ok) * n0 - popc(from & cw) - popc(from & ce);
+            const u64 rest = two & ~ok;
+            if (rest) {
+                u32 at = emit.take(popc(rest));
+                each_square(rest, [&](int t) {
+                    emit.put(at++, cmove(t - 2 * PUSH, t, MF_DOUBLE), PC_PAWN | (((epf >> t) & 1ull) ? PC_EP_FLAG : 0u));
+                });
+            }
+        }
+        // captures: a pawn captured there attacks the capturing pawn itself,
+        // which its own moves (w) already hold; the pawn on the other side loses it
+        {
+            const u64 ok = xw & ~(no | full()) & ~cap_w<S>(stay | seen);
+            const u64 from = S ? ok << 9 : ok >> 7;
+            reach(ok);
+            sum += popc(ok) * n0 - popc(from & cw);
+            const u64 rest = xw & ~ok;
+            if (rest) {
+                u32 at = emit.take(popc(rest) + 3 * popc(rest & BACK_RANKS));
+                each_square(rest, [&](int t) { put_pawn(emit, at, t - CW, t, 0); });
+            }
+        }
+        {
+            const u64 ok = xe & ~(no | full()) & ~cap_e<S>(stay | seen);
+            const u64 from = S ? ok << 7 : ok >> 9;
+            reach(ok);
+            sum += popc(ok) * n0 - popc(from & ce);
+            const u64 rest = xe & ~ok;
+            if (rest) {
+                u32 at = emit.take(popc(rest) + 3 * popc(rest & BACK_RANKS));
+                each_square(rest, [&](int t) { put_pawn(emit, at, t - CE, t, 0); });
+            }
+        }
+    }
+    emit_castles_ep<S>(b, f, [&](u16 mv, u32 pc) { emit.put(emit.take(1), mv, pc); });
+
+    // the corrections of the squares reached
+    auto planes = [&](u64 x, u32 unit) {
+        sum += unit * (popc(x & g0) - popc(x & w0)) + (2 * unit) * (popc(x & g1) - popc(x & w1)) +
+               (4 * unit) * (popc(x & g2) - popc(x & w2)) - (8 * unit) * popc(x & w3);
+    };
+    planes(m0, 1);
+    planes(m1, 2);
+    planes(m2, 4);
+    return sum;
+}
+
+}  // namespace pg

@@ -132,6 +132,17 @@ int build_tables(HostTables& t)
         t.pawn_checks[0][s] = ((b << 9) & not_a) | ((b << 7) & not_h);  // black pawns above a white king
         t.pawn_checks[1][s] = ((b >> 7) & not_a) | ((b >> 9) & not_h);  // white pawns below a black king
     }
+    // squares between two squares of one line: the step from one to the other
+    for (int a = 0; a < 64; a++)
+        for (int c = 0; c < 64; c++) {
+            const int dr = (c >> 3) - (a >> 3), df = (c & 7) - (a & 7);
+            u64 m = 0;
+            if (a != c && (dr == 0 || df == 0 || dr == df || dr == -df)) {
+                const int step = 8 * ((dr > 0) - (dr < 0)) + ((df > 0) - (df < 0));
+                for (int s = a + step; s != c; s += step) m |= 1ull << s;
+            }
+            t.between[a][c] = m;
+        }
     return 0;
 }
 
