@@ -98,45 +98,66 @@ struct QEmit {
     }
 };
 
-// reply_sum's emitter for the leaf: entries are reserved from the CTA's
-// counter, and dropped (only counted) beyond the queue's end; the landing
-// piece goes to bits 25-28 as in QEmit
-template <int QCAP> struct QTake {
-    u32* q;
-    u32* queued;
-    u32 tag, taken;
-    __device__ __forceinline__ u32 take(u32 k)
+// reply_sum's emitters for the leaf
+
+// the queued moves of one thread, in a column of CAP words of its own in shared
+// memory (interleaved over the threads, STRIDE = threads) or local memory: the
+// moves to make from its start, the king recounts from its end.  Moves that do
+// not fit are only counted.
+template <int STRIDE, int CAP> struct QColumn {
+    u32* col;
+    u32 tag, made, kings, eps;  // made counts the en-passant children (eps) too
+    __device__ __forceinline__ void put(u32 ent)
     {
-        taken += k;
-        return atomicAdd(queued, k);
+        if (made < (u32)CAP) col[made * STRIDE] = tag + ent;
+        made++;
     }
-    __device__ __forceinline__ void put(u32 at, u16 m, u32 piece)
+    __device__ __forceinline__ void put_ep(u32 ent)
     {
-        if (at < (u32)QCAP) q[at] = tag | m | (piece << 25);
+        put(ent);
+        eps++;
+    }
+    __device__ __forceinline__ void sets(u64 rest, u64 by_king, u32 first, u32 mul)
+    {
+        auto half = [&](u32 r, u32 k, u32 f) {
+            for (u32 x = r | k; x; x &= x - 1) {
+                const int t = __ffs(x) - 1;
+                const u32 king = (k >> t) & 1u;
+                const u32 at = king ? (u32)CAP - 1u - kings : made;
+                kings += king;
+                made += 1u - king;
+                if (at < (u32)CAP) col[at * STRIDE] = f + (u32)t * mul;
+            }
+        };
+        half((u32)rest, (u32)by_king, tag + first);
+        half((u32)(rest >> 32), (u32)(by_king >> 32), tag + first + 32u * mul);
     }
 };
 
-// the same moves again at fixed positions: those in [lo, hi) are written
+// the same moves written at fixed positions by a second pass: those in
+// [lo, hi), all kinds in one sequence
 struct QWindow {
     u32* q;
-    u32 pos, lo, hi, tag;
-    __device__ __forceinline__ u32 take(u32 k)
+    u32 pos, lo, hi, tag, kings;
+    __device__ __forceinline__ void put(u32 ent)
     {
-        const u32 at = pos;
-        pos += k;
-        return at;
+        if (pos >= lo && pos < hi) q[pos - lo] = tag + ent;
+        pos++;
     }
-    __device__ __forceinline__ void put(u32 at, u16 m, u32 piece)
+    __device__ __forceinline__ void put_ep(u32 ent) { put(ent); }
+    __device__ __forceinline__ void sets(u64 rest, u64 by_king, u32 first, u32 mul)
     {
-        if (at >= lo && at < hi) q[at - lo] = tag | m | (piece << 25);
+        each_square(rest, [&](int t) { put(first + (u32)t * mul); });
+        each_square(by_king, [&](int t) { put((first + (u32)t * mul) | Q_KING); });
+        kings += popc(by_king);
     }
 };
 // one node's part of a queue window (rare: a CTA with more children than its
 // queue holds), out of line so that the leaf keeps one copy of reply_sum
 template <int S> __device__ __noinline__ void queue_window(const Pos& b, u32* q, u32 off, u32 lo, u32 hi, u32 tag)
 {
-    QWindow e{q, off, lo, hi, tag};
-    reply_sum<S>(b, ks_facts<S>(b), e);
+    QWindow e{q, off, lo, hi, tag, 0u};
+    reply_sum<S>(b, e);
 }
 
 struct ArrEmit {
@@ -279,11 +300,24 @@ __global__ void k_count_level(LevelView lv, u32 start, u32 n, u32* __restrict__ 
     count_level_body<S, SL>(lv, start, n, cnt, min_rem);
 }
 
+constexpr int LEAF_COLUMN = 48;  // queued moves a thread holds before they are gathered
+
 template <class SL, int T, int QCAP> struct BlockSmem {
     static constexpr int tables = table_smem_bytes<SL>();
     static constexpr int boards = T * (int)sizeof(Pos);
     static constexpr int queue = QCAP * 4;
     static constexpr int bytes = tables + boards + queue + T * 4 + T;
+};
+
+// the leaf's: no remaining depths, but the threads' columns (in local memory
+// where the byte-lookup policy's tables leave no room)
+template <class SL, int T, int QCAP> struct LeafSmem {
+    static constexpr int tables = table_smem_bytes<SL>();
+    static constexpr int boards = T * (int)sizeof(Pos);
+    static constexpr int queue = QCAP * 4;
+    static constexpr bool column_shared = SL::kId != 2;
+    static constexpr int column_at = tables + boards + queue + T * 4;
+    static constexpr int bytes = column_at + (column_shared ? T * LEAF_COLUMN * 4 : 0);
 };
 
 // register cap: at least PG_LEAF_MIN_WARPS resident warps per SM
@@ -342,16 +376,19 @@ __device__ __forceinline__ void expand_body(const LevelView& in, u32 start, u32 
         const u32 total = (u32)(offs[c1] - chunk_off);
         const u64 chunk_out = chunk_off - out_base;
         Pos bd{0, 0, 0, 0, 0, 0};
-        u32 c = 0, off = 0;
+        u32 c = 0, off = 0, grp = 0;
+        unsigned char rem = 0;
         if (i < c1) {
             const u64 o0 = offs[i];
             c = (u32)(offs[i + 1] - o0);
             off = (u32)(o0 - chunk_off);
             bd = load_board(in, start + i);
-            sg[tid] = in.grp[start + i];
-            sr[tid] = in.rem[start + i];
+            grp = in.grp[start + i];
+            rem = in.rem[start + i];
         }
         sb[tid] = bd;
+        sg[tid] = grp;  // every slot holds a group in range, whatever a queue entry names
+        sr[tid] = rem;
         for (u32 lo = 0; lo < total; lo += QCAP) {
             const u32 hi = min(lo + (u32)QCAP, total);
             if (c && off < hi && off + c > lo) {

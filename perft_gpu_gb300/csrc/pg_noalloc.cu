@@ -200,10 +200,11 @@ LevelView from_node(const LevelView& lv, u64 k)
 template <int S>
 void launch_leaf_na(const LevelView& lv, u32 start, u32 n, u64* out, u32* ticket, cudaStream_t st, int sms)
 {
-    constexpr int Q = NA_T * 32;
-    using L = BlockSmem<SlKS, NA_T, Q>;
-    auto fn = k_leaf<S, SlKS, NA_T, Q>;
-    fn<<<grid_of((const void*)fn, NA_T, L::bytes, n, sms), NA_T, L::bytes, st>>>(lv, start, n, out, ticket, 2u);
+    constexpr int T = 128, Q = T * 24;
+    using L = LeafSmem<SlKS, T, Q>;
+    static_assert(L::bytes <= 48 * 1024, "dynamic shared memory above the default limit");
+    auto fn = k_leaf<S, SlKS, T, Q>;
+    fn<<<grid_of((const void*)fn, T, L::bytes, n, sms), T, L::bytes, st>>>(lv, start, n, out, ticket, 2u);
 }
 
 template <int S>

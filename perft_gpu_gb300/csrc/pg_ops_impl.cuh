@@ -9,14 +9,14 @@
 namespace pg {
 namespace {
 
-// shared-memory queue entries per CTA: 64 per thread hold the children of
-// a CTA's nodes in one window even for positions with ~50 moves (the leaf
-// kernel's first window generates from the count's analysis; a second
-// window makes it again and runs a second copy of the hot loop); the
-// byte-lookup policy gives 158 KB of the CTA's shared memory to its tables
-// and keeps 8
+// shared-memory queue entries per CTA.  The leaf queues the moves that are not
+// counted in sets, about 10 a node: 24 per thread hold them in one window.
+// The expansion queues every move: 64 per thread hold the children of nodes
+// with ~50 moves.  The byte-lookup policy gives 158 KB of the CTA's shared
+// memory to its tables and keeps 8.
 template <class SL, int T> struct QcapFor {
-    static constexpr int value = SL::kId == 2 ? T * 8 : T * 64;
+    static constexpr int leaf = SL::kId == 2 ? T * 8 : T * 24;
+    static constexpr int expand = SL::kId == 2 ? T * 8 : T * 64;
 };
 
 inline int occupancy_grid(const void* fn, int T, int smem, u64 items, int num_sms)
@@ -46,8 +46,8 @@ template <int S, class SL, int T>
 cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem, cudaStream_t st,
                    int sms)
 {
-    constexpr int Q = QcapFor<SL, T>::value;
-    using L = BlockSmem<SL, T, Q>;
+    constexpr int Q = QcapFor<SL, T>::leaf;
+    using L = LeafSmem<SL, T, Q>;
     auto fn = k_leaf<S, SL, T, Q>;
     static cudaError_t attr = set_smem(fn, L::bytes);
     if (attr) return attr;
@@ -60,7 +60,7 @@ template <int S, class SL, int T>
 cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* offs, const LevelView& out, u32* ticket,
                      cudaStream_t st, int sms)
 {
-    constexpr int Q = QcapFor<SL, T>::value;
+    constexpr int Q = QcapFor<SL, T>::expand;
     using L = BlockSmem<SL, T, Q>;
     auto fn = k_expand<S, SL, T, Q>;
     static cudaError_t attr = set_smem(fn, L::bytes);

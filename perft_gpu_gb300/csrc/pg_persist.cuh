@@ -36,7 +36,8 @@ namespace pg {
 
 constexpr u64 PERSIST_BARRIER_NS = 60ull * 1000 * 1000 * 1000;  // 60 s of global time per barrier
 constexpr int PERSIST_T = PERSIST_CTA;
-constexpr int PERSIST_Q = PERSIST_T * 64;                        // queue entries per CTA (as k_leaf)
+constexpr int PERSIST_Q = PERSIST_T * 64;                        // queue entries per CTA (as k_expand)
+constexpr int PERSIST_LEAF_Q = PERSIST_T * 24;                   // and in the leaf phase (as k_leaf)
 constexpr int PERSIST_SCAN_V = 8;                                // counts per thread per scan tile
 constexpr int PERSIST_SCAN_TILE = PERSIST_T * PERSIST_SCAN_V;
 static_assert(PERSIST_SCAN_TILE == (int)PERSIST_SCAN_TILE_NODES, "scan tile known to the host");
@@ -211,7 +212,7 @@ __device__ __forceinline__ void persist_plan(const u64* offs, u32 n, u64 cap, Pl
 template <int S>
 __device__ __forceinline__ void persist_leaf(const PersistArgs& A, int L, u32 start, u32 n, u32* ticket)
 {
-    leaf_body<S, SlKS, PERSIST_T, PERSIST_Q>(A.lv[L], start, n, A.acc, ticket, 2u);
+    leaf_body<S, SlKS, PERSIST_T, PERSIST_LEAF_Q>(A.lv[L], start, n, A.acc, ticket, 2u);
 }
 
 template <int S>
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(PERSIST_T, min_blocks<PERSIST_T>()) k_persist(
 // one CTA per free slot of every SM: all resident, as the barriers need
 inline cudaError_t persist_launch_impl(const PersistArgs& a, cudaStream_t st, int num_sms, int* grid)
 {
-    constexpr int smem = BlockSmem<SlKS, PERSIST_T, PERSIST_Q>::bytes;
+    constexpr int smem = std::max(BlockSmem<SlKS, PERSIST_T, PERSIST_Q>::bytes, LeafSmem<SlKS, PERSIST_T, PERSIST_LEAF_Q>::bytes);
     static_assert(smem <= 48 * 1024, "dynamic shared memory above the default limit");
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, PERSIST_T, smem);

@@ -11,37 +11,44 @@
 //    plain targets times (passed count + correction for the square left), and
 //    over all pieces the corrections for the squares reached, as popcounts of
 //    bit planes (a square's correction in binary, one 64-bit mask per digit);
-//  * every other move (a check, a discovered line, a change of the squares the
-//    king may enter, castling, promotion, en passant, ...) goes to the
-//    emitter, and is made and counted as before.
+//  * after some of them only the opponent king's own moves change otherwise:
+//    they are counted as plain less the king's part, and the emitter gets them
+//    for a recount of the king's moves alone (king_replies);
+//  * every other move (a check, a discovered line, castling, promotion, en
+//    passant, ...) goes to the emitter, and is made and counted as before.
 //
 // A move from f to t by piece X is plain when, with K the opponent's king:
 //  1. K is not attacked on the unmoved board (else no move is plain);
 //  2. f and t change no pin and no check: f is not a blocker whose leaving
 //     opens a line of another mover's slider to K or pins a piece, nor a
 //     pinner; t is not on a line X itself then looks along to K through at most
-//     one opposing piece; t does not unpin or capture a pinned piece;
-//  3. the squares K may enter (and cross when castling) are attacked or not
+//     one opposing piece; t does not unpin or capture a pinned piece; a pinned
+//     slider sees neither f nor t;
+//  3. f and t do not share a line of an opposing slider that sees f, and t is
+//     not a pawn whose own count the square left has already corrected;
+// and the king's replies change too unless
+//  4. the squares K may enter (and cross when castling) are attacked or not
 //     as before: X attacks none of the attacked ones from f alone and none of
 //     the free ones from t, no slider's line through f or t reaches one, and
-//     neither f nor t is next to K or on a castling path;
-//  4. f and t do not share a line of an opposing slider that sees f, and t is
-//     not a piece whose own count the square left has already corrected.
+//     neither f nor t is next to K (nor on a castling path: such a move is made).
 // Then the replies change only by
-//  * the opponent's sliders (pinned ones do not see f or t): the rays that
-//    ended on f run on, the rays that passed t end there;
+//  * the opponent's sliders: the rays that ended on f run on, the rays that
+//    passed t end there;
 //  * its pawns: pushes onto f and t, captures on f and t;
 //  * a captured piece: its own moves go, and the pieces that defend t (sliders,
 //    knights, pawns) gain the recapture.
 // The legality rules enter only through the passed count, whose terms are
 // count_moves_ks1's outside check.
 //
-// What bounds it: integer-ALU issue, as the count of a made child (about 650
-// instructions); the set-wise part costs a node a few children's worth and
-// replaces 71% of its children (batched uneven workload, 34 moves a node).
-// Measured (GB300): 4,096 positions at depths 3..6 in 653 ms against 1,222 ms
-// with every child made and counted; one position at depth 7 in 23.0 against
-// 46.6 ms.
+// What bounds it: integer-ALU issue (66-70% busy in this part; the rest is the
+// latency of dependent instructions and table loads with 16 warps an SM), as
+// the count of a made child (about 900 instructions).  The set-wise part costs
+// a node about 5,500, six children's worth, and replaces 71% of its 34 moves,
+// a king recount (about 150) another 9%.
+// Measured (GB300): 4,096 positions at depths 3..6 in 626 ms, 1,237 ms with
+// every child made and counted; one position at depth 7 in 36.2 against 92.5 ms;
+// with every move that is not plain made and counted, and one emission loop
+// per piece, every 16th of those positions took 37.5 ms of leaf time, now 34.9.
 #pragma once
 #include "pg_movegen.cuh"
 
@@ -56,47 +63,152 @@ struct Planes3 {
     u64 c0, c1, c2;
 };
 
-// How many targets an opposing slider's ray still has beyond each square it
-// passes, and beyond the slider itself (its moves along the ray): 0..7 per
-// square.  v: the attack fill of the sliders along one direction (blockers
-// included), own: the sliders' side (not a target), sl: the sliders.  The run
-// of targets is followed back one step at a time, through empty squares only.
-template <int SH, bool LEFT> __device__ __forceinline__ Planes3 targets_beyond(u64 v, u64 empty, u64 own, u64 sl)
+// How many targets an opposing slider's ray has beyond each square, 0..7: where
+// it passes, what a piece arriving cuts off; at the slider, its moves along the
+// ray; at the other side's piece it ends on, what that piece leaving opens.
+// s: the sliders' attack fill along one direction (blockers included), x: the
+// same from the squares of `blockers` it ends on, own: the sliders' side (not a
+// target), sl: the sliders.  The run of targets is followed back one step at a
+// time, through empty squares only; the opened squares themselves hold nothing.
+template <int SH, bool LEFT>
+__device__ __forceinline__ Planes3 targets_beyond(u64 s, u64 x, u64 empty, u64 own, u64 sl, u64 blockers)
 {
-    const u64 through = v & empty, at = through | sl;
-    auto back = [](u64 x) { return LEFT ? (x >> SH) : (x << SH); };
-    const u64 r1 = back(v & ~own) & at;
+    const u64 through = (s | x) & empty, at = through | sl | (s & blockers), keep = ~(x & empty);
+    auto back = [](u64 y) { return LEFT ? (y >> SH) : (y << SH); };
+    const u64 r1 = back((s | x) & ~own) & at;
     const u64 r2 = back(r1 & through) & at;
     const u64 r3 = back(r2 & through) & at;
     const u64 r4 = back(r3 & through) & at;
     const u64 r5 = back(r4 & through) & at;
     const u64 r6 = back(r5 & through) & at;
     const u64 r7 = back(r6 & through) & at;
-    return Planes3{(r1 & ~r2) | (r3 & ~r4) | (r5 & ~r6) | r7, (r2 & ~r4) | r6, r4};
+    return Planes3{((r1 & ~r2) | (r3 & ~r4) | (r5 & ~r6) | r7) & keep, ((r2 & ~r4) | r6) & keep, r4 & keep};
 }
 
-// a pawn move by target square; on rank 1 or 8 the four promotions, as emit_pawn_sq
-template <class E> __device__ __forceinline__ void put_pawn(E& emit, u32& at, int from, int to, int fl)
+// A queued move: bits 0-15 the move, 16-24 the node's index in its CTA, 25-28
+// the landing piece (PC_*, with PC_EP_FLAG), 29 only the king's replies are
+// recounted.  A set of moves is a mask and the entry of its square 0, each
+// square t adding t x mul: a piece's mask holds target squares (mul 64), a pawn
+// set's the lower of the two squares of each move (mul 65).
+constexpr u32 Q_PIECE_SHIFT = 25;
+constexpr u32 Q_EP = PC_EP_FLAG << Q_PIECE_SHIFT, Q_KING = 1u << 29;
+// a set of pawn moves over the squares of `to`, step = to - from
+template <int STEP> __device__ __forceinline__ u64 pawn_set(u64 to) { return STEP > 0 ? to >> (STEP > 0 ? STEP : 0) : to; }
+template <int STEP> __device__ __forceinline__ constexpr u32 pawn_entry(int flags = 0)
 {
-    auto one = [&](u16 mv, u32 piece) { emit.put(at++, mv, piece); };
-    emit_pawn_sq(one, from, to, fl);
+    return ((u32)flags << 12) | (u32)(STEP > 0 ? STEP * 64 : -STEP);
 }
 
-// The replies to the plain moves of b (S to move; f = ks_facts of b), summed;
-// every other move goes to emit: emit.take(n) reserves n entries and returns
-// the first one's position, emit.put(position, move, landing piece).
-template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b, const KsFacts<S>& f, E& emit)
+// the four promotions to each square of m, from `step` below it
+template <class E> __device__ __forceinline__ void put_promotions(E& emit, u64 m, int step)
+{
+    if (!m) return;
+    auto put = [&](u16 mv, u32 piece) { emit.put((u32)mv | (piece << Q_PIECE_SHIFT)); };
+    each_square(m, [&](int t) { emit_pawn_sq(put, t - step, t, 0); });
+}
+
+// The king's moves of the side to move next (1 - S) after S's move mv on b,
+// when that king is neither checked before nor after it.  piece: as make_child
+template <int S> __device__ __forceinline__ u32 king_replies(const Pos& b, u16 mv, u32 piece)
+{
+    const int from = mv & 63, to = (mv >> 6) & 63;
+    const u64 src = bit64((u32)from), dst = bit64((u32)to);
+    const u32 pc = piece & 7u;
+    const u64 pawns = b.p & INNER;
+    const u64 occ0 = b.k | pawns | b.n | b.bq | b.rq;
+    const u64 mine = (S ? occ0 & ~b.w : b.w) & ~src, own = (S ? b.w : occ0 & ~b.w) & ~dst;
+    const u64 occ = (occ0 & ~src) | dst;
+    const u64 mrq = (b.rq & mine) | ((pc == PC_ROOK || pc == PC_QUEEN) ? dst : 0ull);
+    const u64 mbq = (b.bq & mine) | ((pc == PC_BISHOP || pc == PC_QUEEN) ? dst : 0ull);
+    const u64 mp = (pawns & mine) | (pc == PC_PAWN ? dst : 0ull);
+    const u64 mn = (b.n & mine) | (pc == PC_KNIGHT ? dst : 0ull);
+    const u64 mk = pc == PC_KING ? dst : b.k & mine;
+    const u64 empty = ~occ;
+    const VPro v(empty);
+    u64 thr = v.up(mrq) | v.down(mrq);
+    const RankPro h(occ);
+    thr |= h.east(mrq) | h.west(mrq);
+    const u64 pass = empty & NOT_A & NOT_H;
+    const DPro<9> d9(pass);
+    thr |= d9.up(mbq) | d9.down(mbq);
+    const DPro<7> d7(pass);
+    thr |= d7.up(mbq) | d7.down(mbq);
+    thr |= pawn_attacks<S>(mp) | knight_set(mn) | __ldg(&g_king[sq_of(mk)]);
+    return popc(__ldg(&g_king[sq_of(b.k & own)]) & ~(own | thr));
+}
+
+// The replies to the plain moves of b (S to move), summed, less the king's part
+// where only that is recounted; the other moves go to emit.sets(moves to make,
+// king recounts, entry of square 0, mul) or, one at a time, to emit.put(entry)
+// and emit.put_ep(entry).  emit.kings counts the king recounts.
+template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b, E& emit)
 {
     constexpr int T = 1 - S;
+    KsFacts<S> f;
+    f.pawns = b.p & INNER;
+    f.occ = b.k | f.pawns | b.n | b.bq | b.rq;
+    {
+        const u64 black = f.occ & ~b.w;
+        f.mine = S ? black : b.w;
+        f.theirs = S ? b.w : black;
+    }
+    f.empty = ~f.occ;
     const u64 mine = f.mine, own = f.theirs, occ = f.occ, empty = f.empty, pawns = f.pawns;
     const u64 mrq = b.rq & mine, mbq = b.bq & mine, mp = pawns & mine, mn = b.n & mine, mk = b.k & mine;
+    const u64 orq = b.rq & own, obq = b.bq & own;
+
+    // one propagator chain per line kind for every fill below
+    const VPro v(empty);
+    const RankPro h(occ);
+    const u64 pass = empty & NOT_A & NOT_H;
+    const DPro<9> d9(pass);
+    const DPro<7> d7(pass);
+    // the opponent's sliders, per direction
+    const u64 s0 = v.up(orq), s1 = v.down(orq), s2 = h.east(orq), s3 = h.west(orq);
+    const u64 s4 = d9.up(obq), s5 = d9.down(obq), s6 = d7.up(obq), s7 = d7.down(obq);
+
+    // the mover's side, as in count_moves_ks1: its king is opaque to the fills,
+    // so the square behind it on a checking line is added to the threats
+    {
+        const int ksq = sq_of(mk);
+        f.ksq = ksq;
+        const u64 kr = SlFancy::rook(ksq, occ), kb = SlFancy::bishop(ksq, occ);
+        const u64 kf = kr & file_of(ksq), kd = kb & __ldg(&g_diag[ksq]);
+        const u64 kh = kr ^ kf, ka = kb ^ kd;
+        f.pf = kf & (s0 | s1) & mine;
+        f.pr = kh & (s2 | s3) & mine;
+        f.pd = kd & (s4 | s5) & mine;
+        f.pa = ka & (s6 | s7) & mine;
+        f.pinned = f.pf | f.pr | f.pd | f.pa;
+        const u64 cr = kr & orq, csl = cr | (kb & obq);
+        f.checkers = csl | (__ldg(&g_knight[ksq]) & b.n & own) | (__ldg(&g_pawn_checks[S][ksq]) & pawns & own);
+        u64 cray = 0, behind = 0;
+        if (csl) {
+            const int csq = lsb(csl);
+            cray = __ldg(&g_between[ksq][csq]);
+            for (u64 s = csl; s; s &= s - 1) {
+                const u64 c = lowbit(s);
+                const u64 kray = (c & kf) ? kf : (c & kh) ? kh : (c & kd) ? kd : ka;
+                behind |= kray & (c > mk ? mk - 1ull : ~(mk | (mk - 1ull)));
+            }
+        }
+        f.safe = cray | f.checkers;
+        f.threat = s0 | s1 | s2 | s3 | s4 | s5 | s6 | s7 | behind | pawn_attacks<T>(pawns & own) | knight_set(b.n & own) |
+                   __ldg(&g_king[sq_of(b.k & own)]);
+        const bool in_check = f.checkers != 0;
+        f.chk_all = in_check ? ~0ull : 0ull;
+        f.tgt = several(f.checkers) ? 0ull : (in_check ? f.safe : ~mine);
+    }
+
     const u64 king = b.k & own;
     const int kq = sq_of(king);
     const u64 kr = SlFancy::rook(kq, occ), kb = SlFancy::bishop(kq, occ);
     const u64 ring = __ldg(&g_king[kq]);
 
-    // squares a plain move may not leave / reach, whatever the piece
-    u64 no_f = ring, no_t = ring;
+    // squares a plain move may not leave / reach, whatever the piece; and
+    // those where only the king's own moves change (from / to next to it, a
+    // line opened to or closed from a square it may enter)
+    u64 no_f = 0, no_t = 0, king_f = ring, king_t = ring;
     // the opponent's king attacked with the mover to move: nothing is plain
     if ((kr & mrq) | (kb & mbq) | (__ldg(&g_knight[kq]) & mn) | (__ldg(&g_pawn_checks[T][kq]) & mp) | (ring & mk)) {
         no_f = ~0ull;
@@ -132,12 +244,6 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         }
     }
     const u64 pinned = pf | pr | pd | pa;
-
-    const VPro v(empty);
-    const RankPro h(occ);
-    const u64 pass = empty & NOT_A & NOT_H;
-    const DPro<9> d9(pass);
-    const DPro<7> d7(pass);
 
     // castling squares of the opponent that its own pieces leave open
     u64 path = 0, cross = 0;
@@ -178,29 +284,35 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
             const u64 b4 = d9.down(u0), b5 = d9.up(u0), b6 = d7.down(u0), b7 = d7.up(u0);
             tr = b0 | b1 | b2 | b3;
             tb = b4 | b5 | b6 | b7;
-            no_f |= (a0 & b0) | (a1 & b1) | (a2 & b2) | (a3 & b3) | (a4 & b4) | (a5 & b5) | (a6 & b6) | (a7 & b7);
+            king_f |= (a0 & b0) | (a1 & b1) | (a2 & b2) | (a3 & b3) | (a4 & b4) | (a5 & b5) | (a6 & b6) | (a7 & b7);
         }
         {
             const RankPro g(occ | u1);
-            no_t |= ((a0 & v.down(u1)) | (a1 & v.up(u1)) | (a2 & g.west(u1)) | (a3 & g.east(u1)) | (a4 & d9.down(u1)) |
+            king_t |= ((a0 & v.down(u1)) | (a1 & v.up(u1)) | (a2 & g.west(u1)) | (a3 & g.east(u1)) | (a4 & d9.down(u1)) |
                      (a5 & d9.up(u1)) | (a6 & d7.down(u1)) | (a7 & d7.up(u1))) & empty;
         }
-        // a slider arriving on K's lines checks, or pins the one piece between
-        tr |= SlFancy::rook(kq, occ ^ (kr & own));
-        tb |= SlFancy::bishop(kq, occ ^ (kb & own));
     }
-    const u64 tn = knight_set(u0 | king), tk = king_set(u0);
+    // where a slider checks, or pins the one piece between
+    const u64 xr = SlFancy::rook(kq, occ ^ (kr & own)), xb = SlFancy::bishop(kq, occ ^ (kb & own));
+    const u64 tn = knight_set(u0), tk = king_set(u0);
+    // with a castling path open, a change near the king may change castling too
+    const u64 strict = path ? ~0ull : 0ull;
+    const u32 k0 = popc(u0 & ring);
 
     // ---- the opponent's moves on the unmoved board ----
     const u64 free_ = own & ~pinned;
-    const u64 orq = b.rq & free_, obq = b.bq & free_, op = pawns & free_;
-    u32 n0 = popc(u0 & ring);
-    for (u64 s = pinned & (b.rq | b.bq); s; s &= s - 1) {
+    const u64 op = pawns & free_;
+    u32 n0 = k0;
+    // a pinned slider is filled as if it were free: its moves off the pin line
+    // are taken back, and nothing it sees is plain
+    for (u64 s = pinned & (orq | obq); s; s &= s - 1) {
         const int q = lsb(s);
         const u64 bit = lowbit(s);
-        u64 m = (b.rq & bit) ? SlFancy::rook(q, occ) : 0ull;
-        if (b.bq & bit) m |= SlFancy::bishop(q, occ);
-        n0 += popc(m & ~own & ((pf & bit) ? file_of(kq) : (pr & bit) ? rank_of(kq) : (pd & bit) ? __ldg(&g_diag[kq]) : anti_of(kq)));
+        u64 m = (orq & bit) ? SlFancy::rook(q, occ) : 0ull;
+        if (obq & bit) m |= SlFancy::bishop(q, occ);
+        n0 -= popc(m & ~own & ~((pf & bit) ? file_of(kq) : (pr & bit) ? rank_of(kq) : (pd & bit) ? __ldg(&g_diag[kq]) : anti_of(kq)));
+        no_f |= m;
+        no_t |= m;
     }
     constexpr u64 back_rank = T ? RANK_1 : RANK_8, last_rank = T ? RANK_1 << 8 : RANK_8 >> 8;
     const u64 d1 = push1<T>(op) & empty;
@@ -229,11 +341,11 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
     // w: per square the replies lost when a piece arrives, plus 2: on an empty
     // square the rays cut off, the pushes blocked and (as 1 - x) the pawn
     // captures gained; on an opposing piece its moves and (as 1 - x) the pawn
-    // recaptures gained.  g: the sliders and knights that recapture.
+    // recaptures gained.  On a square of the mover's own, the replies gained when
+    // its piece leaves, plus 2: the rays opened and (as 1 - x) the pawn captures
+    // lost.  The two 2s cancel.  g: the sliders and knights that recapture.
     u64 w0, w1, w2, w3, g0, g1, g2;
     {
-        const u64 s0 = v.up(orq), s1 = v.down(orq), s2 = h.east(orq), s3 = h.west(orq);
-        const u64 s4 = d9.up(obq), s5 = d9.down(obq), s6 = d7.up(obq), s7 = d7.down(obq);
         n0 += popc(s0 & ~own) + popc(s1 & ~own) + popc(s2 & ~own) + popc(s3 & ~own) + popc(s4 & ~own) + popc(s5 & ~own) +
               popc(s6 & ~own) + popc(s7 & ~own);
         // knights: their moves at their squares, and the first two's attacks
@@ -268,10 +380,14 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
             g1 &= own;
             g2 &= own;
         }
-        Planes3 q0 = targets_beyond<8, true>(s0, empty, own, orq), q1 = targets_beyond<8, false>(s1, empty, own, orq);
-        Planes3 q2 = targets_beyond<1, true>(s2, empty, own, orq), q3 = targets_beyond<1, false>(s3, empty, own, orq);
-        Planes3 q4 = targets_beyond<9, true>(s4, empty, own, obq), q5 = targets_beyond<9, false>(s5, empty, own, obq);
-        const Planes3 q6 = targets_beyond<7, true>(s6, empty, own, obq), q7 = targets_beyond<7, false>(s7, empty, own, obq);
+        Planes3 q0 = targets_beyond<8, true>(s0, v.up(s0 & mine), empty, own, orq, mine);
+        Planes3 q1 = targets_beyond<8, false>(s1, v.down(s1 & mine), empty, own, orq, mine);
+        Planes3 q2 = targets_beyond<1, true>(s2, h.east(s2 & mine), empty, own, orq, mine);
+        const Planes3 q3 = targets_beyond<1, false>(s3, h.west(s3 & mine), empty, own, orq, mine);
+        Planes3 q4 = targets_beyond<9, true>(s4, d9.up(s4 & mine), empty, own, obq, mine);
+        const Planes3 q5 = targets_beyond<9, false>(s5, d9.down(s5 & mine), empty, own, obq, mine);
+        const Planes3 q6 = targets_beyond<7, true>(s6, d7.up(s6 & mine), empty, own, obq, mine);
+        const Planes3 q7 = targets_beyond<7, false>(s7, d7.down(s7 & mine), empty, own, obq, mine);
         // knights' and pawns' moves at their own squares, where the slider
         // planes are zero
         q0.c0 |= kc0;
@@ -322,9 +438,10 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         w2 = plane_sum(a2, b2, c);
         c = plane_carry(a2, b2, c);
         w3 = plane_sum(a3, b3, c);
-        no_t |= plane_carry(a3, b3, c);  // 16 or more: not plain
+        const u64 w4 = plane_carry(a3, b3, c);  // 16 or more: not plain
+        no_t |= w4;
+        no_f |= w4;
     }
-    n0 += 2;
 
     // ---- the mover's moves ----
     // m: how many plain moves reach each square (0..7; a square already
@@ -340,118 +457,110 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
     };
     auto full = [&]() { return m0 & m1 & m2; };
 
-    const u64 tgt = f.tgt;
-    const int ksq = f.ksq;
-    const u64 pin_chk = f.pinned & f.chk_all;
-    for (u64 s = mk | (mn & ~f.pinned) | ((mrq | mbq) & ~pin_chk); s; s &= s - 1) {
-        const int q = lsb(s);
-        const u64 bit = lowbit(s);
-        const bool is_k = (mk & bit) != 0, is_n = (mn & bit) != 0, is_r = (mrq & bit) != 0, is_b = (mbq & bit) != 0;
-        const u64 ra = SlFancy::rook(q, occ), ba = SlFancy::bishop(q, occ);
-        const u64 att = is_k ? __ldg(&g_king[q]) : is_n ? __ldg(&g_knight[q]) : ((is_r ? ra : 0ull) | (is_b ? ba : 0ull));
-        u64 to = att & (is_k ? ~(f.threat | mine) : tgt);
-        if (f.pinned & bit)
-            to &= (f.pf & bit) ? file_of(ksq) : (f.pr & bit) ? rank_of(ksq) : (f.pd & bit) ? __ldg(&g_diag[ksq]) : anti_of(ksq);
-        // the square left: pawns that could capture or were blocked there, and
-        // the opposing sliders' rays that run on (t on such a line: not plain)
-        u64 no = no_t | full() | (is_k ? tk : is_n ? tn : ((is_r ? tr : 0ull) | (is_b ? tb : 0ull)));
-        const u64 pawn_att = __ldg(&g_pawn_checks[S][q]) & op;
-        const u64 front = push1<S>(fronts & bit);
-        no |= pawn_att | front;
-        u32 gain = n0 + (front != 0) - popc(pawn_att);
-        for (u64 x = (ra & orq) | (ba & obq); x; x &= x - 1) {
-            const int a = lsb(x);
-            const u64 ab = lowbit(x);
-            const u64 fl = file_of(q), dg = __ldg(&g_diag[q]);
-            const u64 line = (ra & ab) ? ((fl & ab) ? ra & fl : ra & ~fl) : ((dg & ab) ? ba & dg : ba & ~dg);
-            no |= line;
-            gain += popc(line & ~own & (a < q ? ~(bit | (bit - 1)) : bit - 1));
-        }
-        if ((bit & no_f) | (att & u_once)) no = ~0ull;
-        const u64 plain = to & ~no;
-        reach(plain);
-        sum += popc(plain) * gain;
-        const u64 rest = to & no;
-        if (rest) {
-            u32 at = emit.take(popc(rest));
-            const u32 pc = is_k ? PC_KING : is_n ? PC_KNIGHT : is_r ? (is_b ? PC_QUEEN : PC_ROOK) : PC_BISHOP;
-            each_square(rest, [&](int t) { emit.put(at++, cmove(q, t, 0), pc); });
-        }
-    }
-
-    // pawns, by target square; from = to - step
+    // pawns, by target square
     constexpr int PUSH = S ? -8 : 8, CW = S ? -9 : 7, CE = S ? -7 : 9;
-    const u64 fp = mp & ~f.pinned;
-    const u64 pin_ok = ~f.chk_all;
-    const u64 x1 = push1<S>(fp | (mp & f.pf & pin_ok)) & empty;
-    const u64 one = x1 & tgt;
-    const u64 two = push1<S>(x1 & double_rank<S>() & ~f.safe) & empty & tgt;
-    const u64 xw = cap_w<S>(fp | (mp & (S ? f.pd : f.pa) & pin_ok)) & own & tgt;
-    const u64 xe = cap_e<S>(fp | (mp & (S ? f.pa : f.pd) & pin_ok)) & own & tgt;
     {
-        // squares a pawn may not leave, those where an opposing slider's ray
-        // that runs on (pushes: not along the file) is not corrected for, and
-        // squares it may not reach
-        const u64 stay = no_f | cap_w<T>(u_once) | cap_e<T>(u_once) | fronts;
-        const u64 sv0 = v.up(orq) | v.down(orq);
-        const u64 so2 = h.east(orq), so3 = h.west(orq), so4 = d9.up(obq), so5 = d9.down(obq), so6 = d7.up(obq), so7 = d7.down(obq);
-        const u64 seen = sv0 | so2 | so3 | so4 | so5 | so6 | so7;
-        const u64 no = no_t | pawn_attackers_of<T>(u0 | king) | BACK_RANKS;
+        const u64 tgt = f.tgt;
+        const u64 fp = mp & ~f.pinned;
+        const u64 pin_ok = ~f.chk_all;
+        const u64 x1 = push1<S>(fp | (mp & f.pf & pin_ok)) & empty;
+        const u64 one = x1 & tgt;
+        const u64 two = push1<S>(x1 & double_rank<S>() & ~f.safe) & empty & tgt;
+        const u64 xw = cap_w<S>(fp | (mp & (S ? f.pd : f.pa) & pin_ok)) & own & tgt;
+        const u64 xe = cap_e<S>(fp | (mp & (S ? f.pa : f.pd) & pin_ok)) & own & tgt;
+        // squares a pawn may not leave (fronts: it blocks an opposing pawn), may
+        // not leave along the file or a diagonal an opposing slider sees it on
+        // (t on that line), and may not reach; near: only the king's moves change
+        const u64 near_f = king_f | cap_w<T>(u_once) | cap_e<T>(u_once);
+        const u64 near_t = king_t | pawn_attackers_of<T>(u0);
+        const u64 no = no_t | pawn_attackers_of<T>(king) | BACK_RANKS | (near_t & strict);
+        const u64 stay = no_f | fronts | (near_f & strict);
+        // the replies that leaving the squares of x gives, plus 2 a square
+        auto leave = [&](u64 x) { return popc(x & w0) + 2 * popc(x & w1) + 4 * popc(x & w2) + 8 * popc(x & w3); };
         {
-            const u64 ok = one & ~(no | full()) & ~push1<S>(stay | sv0);
-            const u64 from = push1<T>(ok);
+            const u64 ok = one & ~no & ~push1<S>(stay | s0 | s1);
+            const u64 from = push1<T>(ok), by_king = ok & (near_t | push1<S>(near_f));
             reach(ok);
-            const u64 nown = ~own;
-            sum += popc(ok) * n0 - popc(from & cw) - popc(from & ce) + popc(h.east(so2 & from) & nown) +
-                   popc(h.west(so3 & from) & nown) + popc(d9.up(so4 & from) & nown) + popc(d9.down(so5 & from) & nown) +
-                   popc(d7.up(so6 & from) & nown) + popc(d7.down(so7 & from) & nown);
-            const u64 rest = one & ~ok;
-            if (rest) {
-                u32 at = emit.take(popc(rest) + 3 * popc(rest & BACK_RANKS));
-                each_square(rest, [&](int t) { put_pawn(emit, at, t - PUSH, t, 0); });
-            }
+            sum += popc(ok) * n0 + leave(from);
+            const u64 rest = one & ~ok & ~BACK_RANKS;
+            emit.sets(pawn_set<PUSH>(rest), pawn_set<PUSH>(by_king), pawn_entry<PUSH>(), 65u);
+            put_promotions(emit, one & BACK_RANKS, PUSH);
         }
         {
             const u64 ep = (pawns & own);
             const u64 epf = two & (east1(ep) | west1(ep));
-            const u64 ok = two & ~(no | full() | epf) & ~push1<S>(push1<S>(stay | seen));
-            const u64 from = push1<T>(push1<T>(ok));
+            const u64 ok = two & ~(no | epf) & ~push1<S>(push1<S>(stay | s0 | s1));
+            const u64 from = push1<T>(push1<T>(ok)), by_king = ok & (near_t | push1<S>(push1<S>(near_f)));
             reach(ok);
-            sum += popc(ok) * n0 - popc(from & cw) - popc(from & ce);
-            const u64 rest = two & ~ok;
-            if (rest) {
-                u32 at = emit.take(popc(rest));
-                each_square(rest, [&](int t) {
-                    emit.put(at++, cmove(t - 2 * PUSH, t, MF_DOUBLE), PC_PAWN | (((epf >> t) & 1ull) ? PC_EP_FLAG : 0u));
-                });
-            }
+            sum += popc(ok) * n0 + leave(from);
+            const u64 rest = two & ~ok & ~epf;
+            emit.sets(pawn_set<2 * PUSH>(rest), pawn_set<2 * PUSH>(by_king), pawn_entry<2 * PUSH>(MF_DOUBLE), 65u);
+            each_square(epf, [&](int t) { emit.put_ep(cmove(t - 2 * PUSH, t, MF_DOUBLE) | Q_EP); });
         }
         // captures: a pawn captured there attacks the capturing pawn itself,
-        // which its own moves (w) already hold; the pawn on the other side loses it
+        // which its own moves (w at its square) already hold
         {
-            const u64 ok = xw & ~(no | full()) & ~cap_w<S>(stay | seen);
-            const u64 from = S ? ok << 9 : ok >> 7;
+            const u64 ok = xw & ~no & ~cap_w<S>(stay | (S ? s4 | s5 : s6 | s7));
+            const u64 from = S ? ok << 9 : ok >> 7, by_king = ok & (near_t | cap_w<S>(near_f));
             reach(ok);
-            sum += popc(ok) * n0 - popc(from & cw);
-            const u64 rest = xw & ~ok;
-            if (rest) {
-                u32 at = emit.take(popc(rest) + 3 * popc(rest & BACK_RANKS));
-                each_square(rest, [&](int t) { put_pawn(emit, at, t - CW, t, 0); });
-            }
+            sum += popc(ok) * n0 + leave(from) + popc(from & ce);
+            const u64 rest = xw & ~ok & ~BACK_RANKS;
+            emit.sets(pawn_set<CW>(rest), pawn_set<CW>(by_king), pawn_entry<CW>(), 65u);
+            put_promotions(emit, xw & BACK_RANKS, CW);
         }
         {
-            const u64 ok = xe & ~(no | full()) & ~cap_e<S>(stay | seen);
-            const u64 from = S ? ok << 7 : ok >> 9;
+            const u64 ok = xe & ~no & ~cap_e<S>(stay | (S ? s6 | s7 : s4 | s5));
+            const u64 from = S ? ok << 7 : ok >> 9, by_king = ok & (near_t | cap_e<S>(near_f));
             reach(ok);
-            sum += popc(ok) * n0 - popc(from & ce);
-            const u64 rest = xe & ~ok;
-            if (rest) {
-                u32 at = emit.take(popc(rest) + 3 * popc(rest & BACK_RANKS));
-                each_square(rest, [&](int t) { put_pawn(emit, at, t - CE, t, 0); });
-            }
+            sum += popc(ok) * n0 + leave(from) + popc(from & cw);
+            const u64 rest = xe & ~ok & ~BACK_RANKS;
+            emit.sets(pawn_set<CE>(rest), pawn_set<CE>(by_king), pawn_entry<CE>(), 65u);
+            put_promotions(emit, xe & BACK_RANKS, CE);
         }
     }
-    emit_castles_ep<S>(b, f, [&](u16 mv, u32 pc) { emit.put(emit.take(1), mv, pc); });
+    emit_castles_ep<S>(b, f, [&](u16 mv, u32 pc) { emit.put((u32)mv | (pc << Q_PIECE_SHIFT)); });
+
+    // one piece's moves to the squares of `to`: no / near: the squares where they
+    // are not plain / only the king's moves change
+    auto piece = [&](int q, u64 bit, u64 to, u64 att, u64 no, u64 near, u32 pc) {
+        const bool hi = q >= 32;
+        const u32 sq = q & 31;
+        auto at = [&](u64 x) { return ((hi ? (u32)(x >> 32) : (u32)x) >> sq) & 1u; };
+        const u64 pawn_att = __ldg(&g_pawn_checks[S][q]) & op, front = push1<S>(fronts & bit);
+        no |= no_t | full() | pawn_att | front;
+        near |= king_t;
+        if ((bit & king_f) | (att & u_once)) near = ~0ull;
+        no |= near & strict;
+        if (bit & no_f) no = ~0ull;
+        const u64 plain = to & ~no, by_king = plain & near, rest = to & no;
+        reach(plain);
+        sum += popc(plain) * (n0 + (front != 0) + at(w0) + 2 * at(w1) + 4 * at(w2) + 8 * at(w3));
+        emit.sets(rest, by_king, (u32)q | (pc << Q_PIECE_SHIFT), 64u);
+    };
+    const u64 sv = s0 | s1, sh = s2 | s3, sd = s4 | s5, sa = s6 | s7;
+    // the king and the knights
+    for (u64 s = mk | (mn & ~f.pinned); s; s &= s - 1) {
+        const int q = lsb(s);
+        const u64 bit = lowbit(s);
+        const bool is_k = (mk & bit) != 0;
+        const u64 att = is_k ? __ldg(&g_king[q]) : __ldg(&g_knight[q]);
+        // a king that an opposing slider sees (in check) may stay on its line
+        const u64 no = is_k ? ((bit & (sv | sh | sd | sa)) ? ~0ull : 0ull) : __ldg(&g_knight[kq]);
+        piece(q, bit, att & (is_k ? ~(f.threat | mine) : f.tgt), att, no, is_k ? tk : tn, is_k ? PC_KING : PC_KNIGHT);
+    }
+    for (u64 s = (mrq | mbq) & ~(f.pinned & f.chk_all); s; s &= s - 1) {
+        const int q = lsb(s);
+        const u64 bit = lowbit(s);
+        const bool is_r = (mrq & bit) != 0, is_b = (mbq & bit) != 0;
+        const u64 fl = file_of(q), rk = rank_of(q), dg = __ldg(&g_diag[q]), an = anti_of(q);
+        const u64 att = (is_r ? SlFancy::rook(q, occ) : 0ull) | (is_b ? SlFancy::bishop(q, occ) : 0ull);
+        u64 to = att & f.tgt;
+        if (f.pinned & bit) to &= (f.pf & bit) ? fl : (f.pr & bit) ? rk : (f.pd & bit) ? dg : an;
+        // along a line on which an opposing slider sees it
+        const u64 no = (is_r ? xr : 0ull) | (is_b ? xb : 0ull) | ((sv & bit) ? fl : 0ull) | ((sh & bit) ? rk : 0ull) |
+                       ((sd & bit) ? dg : 0ull) | ((sa & bit) ? an : 0ull);
+        piece(q, bit, to, att, no, (is_r ? tr : 0ull) | (is_b ? tb : 0ull), is_r ? (is_b ? PC_QUEEN : PC_ROOK) : PC_BISHOP);
+    }
 
     // the corrections of the squares reached
     auto planes = [&](u64 x, u32 unit) {
@@ -461,7 +570,7 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
     planes(m0, 1);
     planes(m1, 2);
     planes(m2, 4);
-    return sum;
+    return (u64)(sum - emit.kings * k0);
 }
 
 }  // namespace pg

@@ -42,13 +42,23 @@ static int cudaStreamSynchronize(int) { return 0; }
 namespace pg {
 unsigned char pg_dyn_smem[16];
 
-struct Moves {
+struct Moves {  // the emitter of both generators
     u16 mv[4096];
     u32 pc[4096];
-    u32 n = 0;
-    void operator()(u16 m, u32 piece) { put(take(1), m, piece); }
-    u32 take(u32 k) { u32 at = n; n += k; return at; }
-    void put(u32 at, u16 m, u32 piece) { mv[at] = m; pc[at] = piece; }
+    u32 n = 0, kings = 0;
+    u32 king_entry[4096];
+    void operator()(u16 m, u32 piece) { put((u32)m | (piece << Q_PIECE_SHIFT)); }
+    void put(u32 ent)
+    {
+        mv[n] = (u16)ent;
+        pc[n++] = (ent >> Q_PIECE_SHIFT) & 15u;
+    }
+    void put_ep(u32 ent) { put(ent); }
+    void sets(u64 rest, u64 by_king, u32 first, u32 mul)
+    {
+        each_square(rest, [&](int t) { put(first + (u32)t * mul); });
+        each_square(by_king, [&](int t) { king_entry[kings++] = first + (u32)t * mul; });
+    }
 };
 
 template <int S> static u64 replies(const Pos& b, const Moves& e)
@@ -59,19 +69,20 @@ template <int S> static u64 replies(const Pos& b, const Moves& e)
         make_child<S>(c, e.mv[i], e.pc[i]);
         sum += count_moves_ks1<1 - S>(c);
     }
+    for (u32 i = 0; i < e.kings; i++)
+        sum += king_replies<S>(b, (u16)e.king_entry[i], (e.king_entry[i] >> Q_PIECE_SHIFT) & 15u);
     return sum;
 }
 
 template <int S> static void both_ways(const Pos& b, u64* split, u64* made, u32* moves, u32* queued)
 {
-    const KsFacts<S> f = ks_facts<S>(b);
     Moves all, rest;
-    gen_from_facts<S>(b, f, all);
+    gen_from_facts<S>(b, ks_facts<S>(b), all);
     *made = replies<S>(b, all);
-    *split = reply_sum<S>(b, f, rest);
+    *split = reply_sum<S>(b, rest);
     *split += replies<S>(b, rest);
     *moves = all.n;
-    *queued = rest.n;
+    *queued = rest.n + rest.kings;
 }
 }  // namespace pg
 
