@@ -100,7 +100,7 @@ typedef struct pg_opts {
     int graph;                   /* replay the call's launch sequence from a captured CUDA graph */
     pg_stats *stats;             /* optional out */
     int persistent;              /* the whole batch as one persistent cooperative launch that walks
-                                    the levels and chunks on the device (Kogge-Stone sliders, 128-thread
+                                    the levels and chunks on the device (Kogge-Stone sliders, 256-thread
                                     CTAs, two-ply leaf; no TT): the reference's device-side driver,
                                     perft_bb.h:1143-1220, without dynamic parallelism */
 } pg_opts;

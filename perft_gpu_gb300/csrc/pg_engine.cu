@@ -717,6 +717,7 @@ static int perft_batch_graph_locked(const Pos* d_pos, const unsigned char* d_dep
 static int prepare_persist(u32 n, int maxd, PersistArgs& A)
 {
     Engine& E = engine();
+    PG_CUDA(persist_setup());
     memset(&A, 0, sizeof(A));
     const int deepest = std::min(std::max(maxd - 2, 0), MAX_LEVELS - 1);
     const u64 capmax = level_cap_max();

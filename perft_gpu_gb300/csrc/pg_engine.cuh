@@ -88,9 +88,15 @@ struct PersistArgs {
     PersistCtl* ctl;
     u32* err;
 };
-// the persistent launch (Kogge-Stone translation unit); *grid = CTAs launched
+// the persistent launch (Kogge-Stone translation unit); *grid = CTAs launched.
+// persist_setup allows the kernel its shared memory (once, outside a capture).
+cudaError_t persist_setup();
 cudaError_t persist_launch(const PersistArgs& a, cudaStream_t st, int num_sms, int* grid);
-constexpr int PERSIST_CTA = 128;  // threads per CTA of the persistent launch
+// threads per CTA of the persistent launch: two CTAs of 256 an SM.  The leaf
+// phase's code is larger than the instruction caches near the schedulers, so
+// warps in step share its fetches: the batched workload's every 16th position
+// took 49.5 ms with four CTAs of 128, 38.0 with two of 256, 39.3 with one of 512
+constexpr int PERSIST_CTA = 256;
 constexpr u32 PERSIST_SCAN_TILE_NODES = 1024;  // counts per scan tile of the persistent launch
 
 // one captured batch (see perft_batch_graph_locked)

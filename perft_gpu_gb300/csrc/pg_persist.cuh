@@ -30,6 +30,8 @@
 #pragma once
 #include <cuda/atomic>
 
+#include <algorithm>
+
 #include "pg_kernels.cuh"
 
 namespace pg {
@@ -38,7 +40,7 @@ constexpr u64 PERSIST_BARRIER_NS = 60ull * 1000 * 1000 * 1000;  // 60 s of globa
 constexpr int PERSIST_T = PERSIST_CTA;
 constexpr int PERSIST_Q = PERSIST_T * 64;                        // queue entries per CTA (as k_expand)
 constexpr int PERSIST_LEAF_Q = PERSIST_T * 24;                   // and in the leaf phase (as k_leaf)
-constexpr int PERSIST_SCAN_V = 8;                                // counts per thread per scan tile
+constexpr int PERSIST_SCAN_V = 4;                                // counts per thread per scan tile
 constexpr int PERSIST_SCAN_TILE = PERSIST_T * PERSIST_SCAN_V;
 static_assert(PERSIST_SCAN_TILE == (int)PERSIST_SCAN_TILE_NODES, "scan tile known to the host");
 
@@ -347,13 +349,21 @@ __global__ void __launch_bounds__(PERSIST_T, min_blocks<PERSIST_T>()) k_persist(
     }
 }
 
+constexpr int PERSIST_SMEM = std::max(BlockSmem<SlKS, PERSIST_T, PERSIST_Q>::bytes, LeafSmem<SlKS, PERSIST_T, PERSIST_LEAF_Q>::bytes);
+inline cudaError_t persist_setup_impl()
+{
+    static const cudaError_t e = cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, PERSIST_SMEM);
+    return e;
+}
+
 // one CTA per free slot of every SM: all resident, as the barriers need
 inline cudaError_t persist_launch_impl(const PersistArgs& a, cudaStream_t st, int num_sms, int* grid)
 {
-    constexpr int smem = std::max(BlockSmem<SlKS, PERSIST_T, PERSIST_Q>::bytes, LeafSmem<SlKS, PERSIST_T, PERSIST_LEAF_Q>::bytes);
-    static_assert(smem <= 48 * 1024, "dynamic shared memory above the default limit");
+    constexpr int smem = PERSIST_SMEM;
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, PERSIST_T, smem);
+    cudaError_t e = persist_setup_impl();
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, PERSIST_T, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorLaunchOutOfResources;
     *grid = per_sm * num_sms;
