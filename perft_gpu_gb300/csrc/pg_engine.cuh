@@ -183,7 +183,8 @@ struct Variant {
 };
 Variant pick_variant(const pg_opts* o);
 u32* next_ticket();
-int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u64* acc);
+// sparse: many nodes of the range are dead
+int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u64* acc, bool sparse = false);
 int launch_expand(const Variant& v, int side, const LevelView& in, u32 start, u32 a, u32 b, const u64* offs,
                   const LevelView& out);
 int launch_count(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u32* cnt);

@@ -300,6 +300,7 @@ __global__ void k_count_level(LevelView lv, u32 start, u32 n, u32* __restrict__ 
     count_level_body<S, SL>(lv, start, n, cnt, min_rem);
 }
 
+constexpr int LEAF_GATHER = 4;  // nodes a thread looks at when the CTA collects the live ones of a sparse level
 constexpr int LEAF_COLUMN = 48;  // queued moves a thread holds before they are gathered
 
 template <class SL, int T, int QCAP> struct BlockSmem {
@@ -316,7 +317,7 @@ template <class SL, int T, int QCAP> struct LeafSmem {
     static constexpr int boards = T * (int)sizeof(Pos);
     static constexpr int queue = QCAP * 4;
     static constexpr bool column_shared = SL::kId != 2;
-    static constexpr int column_at = tables + boards + queue + T * 4;
+    static constexpr int column_at = tables + boards + queue + T * 8;
     static constexpr int bytes = column_at + (column_shared ? T * LEAF_COLUMN * 4 : 0);
 };
 
@@ -332,14 +333,14 @@ template <int T> constexpr int min_blocks() { return (PG_LEAF_MIN_WARPS * 32 + T
 // the compiler keeps more registers for the count (measured 0.5-0.9% faster
 // than calling the inlined function).  LV is LevelView or any type with the
 // same grp[] / rem[] subscripts and a load_board overload.
-template <int S, class SL, int T, int QCAP, class LV>
+template <int S, class SL, int T, int QCAP, bool SPARSE, class LV>
 __device__ __forceinline__ void leaf_body(LV lv, u32 start, u32 n, u64* __restrict__ acc, u32* ticket, u32 max_rem)
 {
     extern __shared__ __align__(16) unsigned char pg_dyn_smem[];
 #include "pg_leaf_body.inc"
 }
 
-template <int S, class SL, int T, int QCAP>
+template <int S, class SL, int T, int QCAP, bool SPARSE>
 __global__ void __launch_bounds__(T, min_blocks<T>()) k_leaf(LevelView lv, u32 start, u32 n, u64* __restrict__ acc, u32* ticket,
                                                             u32 max_rem)
 {

@@ -203,7 +203,7 @@ void launch_leaf_na(const LevelView& lv, u32 start, u32 n, u64* out, u32* ticket
     constexpr int T = 128, Q = T * 24;
     using L = LeafSmem<SlKS, T, Q>;
     static_assert(L::bytes <= 48 * 1024, "dynamic shared memory above the default limit");
-    auto fn = k_leaf<S, SlKS, T, Q>;
+    auto fn = k_leaf<S, SlKS, T, Q, false>;
     fn<<<grid_of((const void*)fn, T, L::bytes, n, sms), T, L::bytes, st>>>(lv, start, n, out, ticket, 2u);
 }
 

@@ -42,13 +42,13 @@ template <class K> cudaError_t set_smem(K fn, int bytes)
                              : cudaSuccess;
 }
 
-template <int S, class SL, int T>
-cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem, cudaStream_t st,
-                   int sms)
+template <int S, class SL, int T, bool SPARSE>
+cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem,
+                   cudaStream_t st, int sms)
 {
     constexpr int Q = QcapFor<SL, T>::leaf;
     using L = LeafSmem<SL, T, Q>;
-    auto fn = k_leaf<S, SL, T, Q>;
+    auto fn = k_leaf<S, SL, T, Q, SPARSE>;
     static cudaError_t attr = set_smem(fn, L::bytes);
     if (attr) return attr;
     const int grid = occupancy_grid((const void*)fn, T, L::bytes, n, sms);
@@ -72,16 +72,19 @@ cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* of
 
 template <class SL>
 cudaError_t leaf_any(int side, int T, const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem,
-                     cudaStream_t st, int sms)
+                     bool sparse, cudaStream_t st, int sms)
 {
+    if (sparse)
+        return side ? leaf_t<1, SL, 256, true>(lv, start, n, acc, ticket, max_rem, st, sms)
+                    : leaf_t<0, SL, 256, true>(lv, start, n, acc, ticket, max_rem, st, sms);
     if (T == 128)
-        return side ? leaf_t<1, SL, 128>(lv, start, n, acc, ticket, max_rem, st, sms)
-                    : leaf_t<0, SL, 128>(lv, start, n, acc, ticket, max_rem, st, sms);
+        return side ? leaf_t<1, SL, 128, false>(lv, start, n, acc, ticket, max_rem, st, sms)
+                    : leaf_t<0, SL, 128, false>(lv, start, n, acc, ticket, max_rem, st, sms);
     if (T == 512)
-        return side ? leaf_t<1, SL, 512>(lv, start, n, acc, ticket, max_rem, st, sms)
-                    : leaf_t<0, SL, 512>(lv, start, n, acc, ticket, max_rem, st, sms);
-    return side ? leaf_t<1, SL, 256>(lv, start, n, acc, ticket, max_rem, st, sms)
-                : leaf_t<0, SL, 256>(lv, start, n, acc, ticket, max_rem, st, sms);
+        return side ? leaf_t<1, SL, 512, false>(lv, start, n, acc, ticket, max_rem, st, sms)
+                    : leaf_t<0, SL, 512, false>(lv, start, n, acc, ticket, max_rem, st, sms);
+    return side ? leaf_t<1, SL, 256, false>(lv, start, n, acc, ticket, max_rem, st, sms)
+                : leaf_t<0, SL, 256, false>(lv, start, n, acc, ticket, max_rem, st, sms);
 }
 
 template <class SL>

@@ -405,7 +405,7 @@ static int run_range_tt(const Variant& v, int L, u32 start, u32 n, int side, int
     k_tt_dedup<<<small_grid(n), 256, 0, E.stream>>>(lb.v, start, n, lt, dd);
     TT_CUDA(cudaGetLastError());
     E.st.launches += 2;
-    if (minrem <= 2) TT_TRY(launch_leaf(v, side, lb.v, start, n, lt.acc));
+    if (minrem <= 2) TT_TRY(launch_leaf(v, side, lb.v, start, n, lt.acc, true));
     if (maxrem < 3) return PG_OK;
     TT_TRY(launch_count(v, side, lb.v, start, n, lb.cnt));
     TT_TRY(launch_scan(lb.cnt, n, lb.offs));

@@ -1,0 +1,55 @@
+"""The two-ply leaf where its queue and its choice of form have their edges:
+CTAs whose queued moves overflow a thread's column and the CTA's queue, partly
+filled CTAs, and levels with many dead nodes around the size from which the
+leaf collects the live ones.  Counts are exact: they equal the oracle's."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# 218 legal moves, and a middlegame with checks and pins on every side
+MANY = "R6R/3Q4/1Q4Q1/4Q3/2Q4Q/Q4Q2/pp1Q4/kBNN1KB1 w - - 0 1"
+SHARP = "r3k2r/p1ppqpb1/bn2pnp1/3PN3/1p2P3/2N2Q1p/PPPBBPPP/R3K2R w KQkq - 0 1"
+
+
+@pytest.fixture(scope="module")
+def orc():
+    import oracle
+    oracle.build()
+    return oracle.Oracle(1)
+
+
+def _copies(pg, fen, n):
+    return np.repeat(pg.boards_array([pg.board_from_fen(fen)]), n)
+
+
+@pytest.mark.parametrize("block", [128, 256, 512])
+@pytest.mark.parametrize("slider", ["ks", "byte"])
+@pytest.mark.parametrize("n", [1, 31, 513])
+def test_leaf_queue_overflows_and_partial_ctas(pg, orc, block, slider, n):
+    for fen in (MANY, SHARP):
+        boards = _copies(pg, fen, n)
+        # every third node one ply shallower, so that nodes of both depths share CTAs
+        depths = np.where(np.arange(n) % 3 == 1, 1, 2).astype(np.uint8)
+        want = {d: orc.perft(orc.fen(fen), d) for d in (1, 2)}
+        got = pg.perft_batch(boards, depths, slider=slider, block_size=block, leaf_plies=2)
+        assert (got == np.array([want[int(d)] for d in depths], dtype=np.uint64)).all()
+
+
+@pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19, (1 << 19) + 1, (1 << 19) + 1500])
+def test_leaf_collects_live_nodes_of_a_sparse_level(pg, orc, n):
+    """n white-to-move nodes of which every second one repeats another."""
+    boards = pg.random_playouts(41, 400000, 2, 60)
+    boards = boards[(boards["pawns"] >> np.uint64(63)) == 0]
+    half = (n + 1) // 2
+    base = boards[np.arange(half) % len(boards)]
+    nodes = np.empty(n, dtype=boards.dtype)
+    nodes[0::2], nodes[1::2] = base, base[:n // 2]
+    got = pg.perft_batch(nodes, np.full(n, 2, np.uint8), use_tt="dedup")
+    distinct, _ = orc.perft_batch(boards[:min(half, len(boards))], np.full(min(half, len(boards)), 2, np.uint8),
+                                  os.cpu_count() or 1)
+    want = distinct[np.arange(half) % len(boards)]
+    assert np.array_equal(got[0::2], want)
+    assert np.array_equal(got[1::2], want[:n // 2])
