@@ -47,6 +47,7 @@ static __device__ u64 g_king[64];
 static __device__ u64 g_diag[64];
 static __device__ u64 g_pawn_checks[2][64];
 static __device__ u64 g_between[64][64];  // squares strictly between two squares of one line
+static __device__ u64 g_behind[64][64];   // the neighbour of the first square away from the second, on their line
 // The count is bound by integer-ALU issue (the ALU pipe ~88-91% busy, the
 // FMA pipe ~10-14%).  Its popcount sums are written as multiply-adds by a 1 the
 // compiler cannot fold (a __constant__ word), so they issue on the FMA pipe
@@ -83,6 +84,7 @@ static inline cudaError_t upload_static_tables(const HostTables& t)
     if ((e = cudaMemcpyToSymbol(g_diag, t.diag, sizeof(t.diag)))) return e;
     if ((e = cudaMemcpyToSymbol(g_pawn_checks, t.pawn_checks, sizeof(t.pawn_checks)))) return e;
     if ((e = cudaMemcpyToSymbol(g_between, t.between, sizeof(t.between)))) return e;
+    if ((e = cudaMemcpyToSymbol(g_behind, t.behind, sizeof(t.behind)))) return e;
     if ((e = cudaMemcpyToSymbol(g_knight, t.knight, sizeof(t.knight)))) return e;
     {
         u64 kt[65];
@@ -562,19 +564,19 @@ __device__ __forceinline__ u32 count_moves_ks1(const Pos& b)
     const u64 cr = kr & trq, cb = kb & tbq;
     const u64 csl = cr | cb;
     const u64 checkers = csl | (__ldg(&g_knight[ksq]) & tn) | (__ldg(&g_pawn_checks[S][ksq]) & tp);
+    // a slider check: the squares between, and the square behind the king on the
+    // line, from tables (a line holds at most one checker; two sliders check
+    // together only after a discovery)
     u64 cray = 0, behind = 0;
-    if (__any_sync(__activemask(), csl != 0)) {
-        const int csq = lsb(csl) & 63;
-        cray = SlFancy::look(cr ? g_magic_rook : g_magic_bishop, csq, occ) & (cr ? kr : kb);
-        for (u64 s = csl; s; s &= s - 1) {
-            const u64 c = s & (0ull - s);
-            const u64 kray = (c & kf) ? kf : (c & kh) ? kh : (c & kd) ? kd : ka;
-            behind |= kray & (c > king ? king - 1ull : ~(king | (king - 1ull)));
-        }
+    if (csl) {
+        const int csq = lsb(csl);
+        cray = __ldg(&g_between[ksq][csq]);
+        behind = __ldg(&g_behind[ksq][csq]);
+        for (u64 s = csl & (csl - 1); s; s &= s - 1) behind |= __ldg(&g_behind[ksq][lsb(s)]);
     }
     const bool in_check = checkers != 0;
     const u64 chk_all = in_check ? ~0ull : 0ull;
-    const u64 safe = (csl ? cray : 0ull) | checkers;
+    const u64 safe = cray | checkers;
     const u64 tgt = several(checkers) ? 0ull : (in_check ? safe : ~mine);
 
     u32 n = 0;

@@ -186,11 +186,7 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         if (csl) {
             const int csq = lsb(csl);
             cray = __ldg(&g_between[ksq][csq]);
-            for (u64 s = csl; s; s &= s - 1) {
-                const u64 c = lowbit(s);
-                const u64 kray = (c & kf) ? kf : (c & kh) ? kh : (c & kd) ? kd : ka;
-                behind |= kray & (c > mk ? mk - 1ull : ~(mk | (mk - 1ull)));
-            }
+            for (u64 s = csl; s; s &= s - 1) behind |= __ldg(&g_behind[ksq][lsb(s)]);
         }
         f.safe = cray | f.checkers;
         f.threat = s0 | s1 | s2 | s3 | s4 | s5 | s6 | s7 | behind | pawn_attacks<T>(pawns & own) | knight_set(b.n & own) |
@@ -468,13 +464,13 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         const u64 two = push1<S>(x1 & double_rank<S>() & ~f.safe) & empty & tgt;
         const u64 xw = cap_w<S>(fp | (mp & (S ? f.pd : f.pa) & pin_ok)) & own & tgt;
         const u64 xe = cap_e<S>(fp | (mp & (S ? f.pa : f.pd) & pin_ok)) & own & tgt;
-        // squares a pawn may not leave (fronts: it blocks an opposing pawn), may
+        // squares a pawn may not leave (fronts: a push stays in an opposing pawn's way), may
         // not leave along the file or a diagonal an opposing slider sees it on
         // (t on that line), and may not reach; near: only the king's moves change
         const u64 near_f = king_f | cap_w<T>(u_once) | cap_e<T>(u_once);
         const u64 near_t = king_t | pawn_attackers_of<T>(u0);
         const u64 no = no_t | pawn_attackers_of<T>(king) | BACK_RANKS | (near_t & strict);
-        const u64 stay = no_f | fronts | (near_f & strict);
+        const u64 stay_x = no_f | (near_f & strict), stay = stay_x | fronts;
         // the replies that leaving the squares of x gives, plus 2 a square
         auto leave = [&](u64 x) { return popc(x & w0) + 2 * popc(x & w1) + 4 * popc(x & w2) + 8 * popc(x & w3); };
         {
@@ -500,19 +496,19 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         // captures: a pawn captured there attacks the capturing pawn itself,
         // which its own moves (w at its square) already hold
         {
-            const u64 ok = xw & ~no & ~cap_w<S>(stay | (S ? s4 | s5 : s6 | s7));
+            const u64 ok = xw & ~no & ~cap_w<S>(stay_x | (S ? s4 | s5 : s6 | s7));
             const u64 from = S ? ok << 9 : ok >> 7, by_king = ok & (near_t | cap_w<S>(near_f));
             reach(ok);
-            sum += popc(ok) * n0 + leave(from) + popc(from & ce);
+            sum += popc(ok) * n0 + leave(from) + popc(from & ce) + popc(from & fronts);
             const u64 rest = xw & ~ok & ~BACK_RANKS;
             emit.sets(pawn_set<CW>(rest), pawn_set<CW>(by_king), pawn_entry<CW>(), 65u);
             put_promotions(emit, xw & BACK_RANKS, CW);
         }
         {
-            const u64 ok = xe & ~no & ~cap_e<S>(stay | (S ? s6 | s7 : s4 | s5));
+            const u64 ok = xe & ~no & ~cap_e<S>(stay_x | (S ? s6 | s7 : s4 | s5));
             const u64 from = S ? ok << 7 : ok >> 9, by_king = ok & (near_t | cap_e<S>(near_f));
             reach(ok);
-            sum += popc(ok) * n0 + leave(from) + popc(from & cw);
+            sum += popc(ok) * n0 + leave(from) + popc(from & cw) + popc(from & fronts);
             const u64 rest = xe & ~ok & ~BACK_RANKS;
             emit.sets(pawn_set<CE>(rest), pawn_set<CE>(by_king), pawn_entry<CE>(), 65u);
             put_promotions(emit, xe & BACK_RANKS, CE);

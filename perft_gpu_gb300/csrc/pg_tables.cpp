@@ -132,16 +132,20 @@ int build_tables(HostTables& t)
         t.pawn_checks[0][s] = ((b << 9) & not_a) | ((b << 7) & not_h);  // black pawns above a white king
         t.pawn_checks[1][s] = ((b >> 7) & not_a) | ((b >> 9) & not_h);  // white pawns below a black king
     }
-    // squares between two squares of one line: the step from one to the other
+    // squares between two squares of one line (the step from one to the other),
+    // and the square behind the first
     for (int a = 0; a < 64; a++)
         for (int c = 0; c < 64; c++) {
             const int dr = (c >> 3) - (a >> 3), df = (c & 7) - (a & 7);
-            u64 m = 0;
+            u64 m = 0, beyond = 0;
             if (a != c && (dr == 0 || df == 0 || dr == df || dr == -df)) {
                 const int step = 8 * ((dr > 0) - (dr < 0)) + ((df > 0) - (df < 0));
                 for (int s = a + step; s != c; s += step) m |= 1ull << s;
+                const int r = (a >> 3) - ((dr > 0) - (dr < 0)), f = (a & 7) - ((df > 0) - (df < 0));
+                if (r >= 0 && r < 8 && f >= 0 && f < 8) beyond = 1ull << (8 * r + f);
             }
             t.between[a][c] = m;
+            t.behind[a][c] = beyond;
         }
     return 0;
 }

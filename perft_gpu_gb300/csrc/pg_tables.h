@@ -28,6 +28,7 @@ struct HostTables {
     u64 king[64];
     u64 diag[64];  // the a1-h8 diagonal through each square
     u64 between[64][64];  // squares strictly between two squares of one line (0 when not aligned)
+    u64 behind[64][64];   // the neighbour of the first square away from the second, on their line
     u64 pawn_checks[2][64];  // squares from which an enemy pawn attacks a king of side s on square q
 };
 
