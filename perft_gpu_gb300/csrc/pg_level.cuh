@@ -11,6 +11,8 @@ namespace pg {
 // transposition-table hit or a duplicate of another node of its level)
 constexpr unsigned char REM_DEAD = 0x80;
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ Pos load_board(const LevelView& lv, u64 i)
 {
     const ulonglong2 a = lv.pl0[i], b = lv.pl1[i], c = lv.pl2[i];
