@@ -272,8 +272,17 @@ static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int mi
         if (!capturing) cudaEventRecord(ev[1], E.stream);
     }
     if (maxrem <= lp) return PG_OK;
-    PG_TRY(launch_count(v, side, lb.v, start, n, lb.cnt));
-    PG_TRY(launch_scan(lb.cnt, n, lb.offs));
+    const u64 cap_next = level_cap_max();
+    const bool fused = n <= PLAN_FUSED_MAX;
+    if (fused) {
+        PG_TICKET(done);
+        PG_CUDA(ops_for(v.slider).count_plan(side, lb.v, start, n, lb.cnt, (u32)lp + 1, lb.offs, cap_next, E.plan_host, done,
+                                             E.err, E.stream));
+        E.st.launches++;
+    } else {
+        PG_TRY(launch_count(v, side, lb.v, start, n, lb.cnt));
+        PG_TRY(launch_scan(lb.cnt, n, lb.offs));
+    }
     std::vector<u32> bnd;
     std::vector<u64> boff;
     if (capturing) {
@@ -286,21 +295,27 @@ static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int mi
         boff = E.rec_off[E.rec_next];
         E.rec_next++;
     } else {
-        const u64 cap_next = level_cap_max();
-        k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_dev, E.err);
-        PG_CUDA(cudaGetLastError());
-        E.st.launches++;
-        u32* perr = (u32*)(E.host_scratch + 192);  // pinned
-        PG_CUDA(cudaMemcpyAsync(E.plan_host, E.plan_dev, sizeof(PlanOut), cudaMemcpyDeviceToHost, E.stream));
-        PG_CUDA(cudaMemcpyAsync(perr, E.err, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
-        PG_CUDA(cudaStreamSynchronize(E.stream));
+        PlanOut& plan = *E.plan_host;  // copied out below: deeper levels reuse the pinned buffer
+        u32 errv = 0;
+        if (fused) {
+            PG_CUDA(cudaStreamSynchronize(E.stream));
+            errv = plan.pad;
+        }
+        if (!fused || (plan.nchunks == 0 && !errv)) {
+            k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_dev, E.err);
+            PG_CUDA(cudaGetLastError());
+            E.st.launches++;
+            u32* perr = (u32*)(E.host_scratch + 192);  // pinned
+            PG_CUDA(cudaMemcpyAsync(E.plan_host, E.plan_dev, sizeof(PlanOut), cudaMemcpyDeviceToHost, E.stream));
+            PG_CUDA(cudaMemcpyAsync(perr, E.err, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
+            PG_CUDA(cudaStreamSynchronize(E.stream));
+            errv = *perr;
+        }
         collect_leaf_timers();
-        const u32 errv = *perr;
         if (errv) {
             set_error("device error flags 0x%x while planning level %d", errv, L);
             return PG_ERR_DEVICE_TIMEOUT;
         }
-        const PlanOut& plan = *E.plan_host;  // copied out: deeper levels reuse the pinned buffer
         bnd.assign(plan.bnd, plan.bnd + plan.nchunks + 1);
         boff.assign(plan.coff, plan.coff + plan.nchunks + 1);
         if (E.plan_mode == PLAN_RECORD) {

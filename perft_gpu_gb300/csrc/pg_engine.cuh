@@ -17,6 +17,7 @@ constexpr int MAX_LEVELS = 16;
 // remaining depth (1), child count (4) and scanned offset (8)
 constexpr u64 LEVEL_NODE_BYTES = 48 + 4 + 1 + 4 + 8;
 constexpr u32 MAX_CHUNKS = 2048;      // greedy chunks planned per expansion
+constexpr u32 PLAN_FUSED_MAX = 8192;  // nodes of a level whose counts, scan and plan are one launch
 constexpr u32 MAX_TICKETS = 1 << 16;  // dynamic-scheduling counters per call
 
 // device error bits (bounded waits and capacity guards set them; no trap)

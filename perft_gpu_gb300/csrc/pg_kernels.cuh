@@ -300,8 +300,72 @@ __global__ void k_count_level(LevelView lv, u32 start, u32 n, u32* __restrict__ 
     count_level_body<S, SL>(lv, start, n, cnt, min_rem);
 }
 
+// Children counts, their scan and the chunk plan of a small level (n up to
+// PLAN_FUSED_MAX) in one launch: the last CTA to finish its counts scans them
+// all.  The plan goes straight to pinned host memory (nchunks 0: the children do
+// not fit one chunk of `cap`, k_plan has to split them; pad: the error bits).
+template <int S, class SL>
+__global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
+                                                    PlanOut* plan, u32* done, const u32* err)
+{
+    stage_tables<SL>();
+    count_level_body<S, SL>(lv, start, n, cnt, min_rem);
+    constexpr int T = 256;
+    __shared__ u32 s_done;
+    __shared__ u64 s_warp[T / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_done = atomicAdd(done, 1u);
+    __syncthreads();
+    if (s_done != gridDim.x - 1) return;
+    __threadfence();
+    const u32 per = (n + T - 1) / T, c0 = min(n, tid * per), c1 = min(n, c0 + per);
+    u64 sum = 0;
+    for (u32 i = c0; i < c1; i++) sum += __ldcg(cnt + i);
+    u64 x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    u64 run = x - sum, total = 0;
+    for (int w = 0; w < T / 32; w++) {
+        if (w < warp) run += s_warp[w];
+        total += s_warp[w];
+    }
+    for (u32 i = c0; i < c1; i++) {
+        offs[i] = run;
+        run += __ldcg(cnt + i);
+    }
+    if (tid == 0) {
+        offs[n] = total;
+        plan->nchunks = total <= cap ? 1u : 0u;
+        plan->pad = *err;
+        plan->total = total;
+        plan->bnd[0] = 0;
+        plan->bnd[1] = n;
+        plan->coff[0] = 0;
+        plan->coff[1] = total;
+    }
+}
+
 constexpr int LEAF_GATHER = 4;  // nodes a thread looks at when the CTA collects the live ones of a sparse level
 constexpr int LEAF_COLUMN = 48;  // queued moves a thread holds before they are gathered
+
+// Nodes per CTA and chunk of a launch over n nodes: the launch's CTAs share a
+// small level, fewer nodes than threads each (whole warps of them once there
+// are that many).  The node phase then runs on some of a CTA's warps and the
+// children, ten (leaf) or thirty (expansion) a node, on all of them, where a full
+// chunk would leave SMs idle and give every thread its nodes' children one after
+// the other.
+__device__ __forceinline__ u32 node_chunk(u32 n, u32 threads)
+{
+    const u32 even = (n + gridDim.x - 1) / gridDim.x;
+    return min(threads, even <= 32u ? even : (even + 31u) & ~31u);
+}
 
 template <class SL, int T, int QCAP> struct BlockSmem {
     static constexpr int tables = table_smem_bytes<SL>();
@@ -366,12 +430,13 @@ __device__ __forceinline__ void expand_body(const LevelView& in, u32 start, u32 
     __shared__ u32 s_chunk;
     const int tid = threadIdx.x;
     const u64 out_base = offs[a];
+    const u32 per = node_chunk(b - a, T);
     for (;;) {
         if (tid == 0) s_chunk = atomicAdd(ticket, 1u);
         __syncthreads();
-        const u64 c0 = (u64)a + (u64)s_chunk * T;
+        const u64 c0 = (u64)a + (u64)s_chunk * per;
         if (c0 >= b) break;
-        const u64 c1 = min(c0 + T, (u64)b);
+        const u64 c1 = min(c0 + per, (u64)b);
         const u64 i = c0 + tid;
         const u64 chunk_off = offs[c0];
         const u32 total = (u32)(offs[c1] - chunk_off);

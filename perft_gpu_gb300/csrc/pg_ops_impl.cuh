@@ -51,7 +51,8 @@ cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket,
     auto fn = k_leaf<S, SL, T, Q, SPARSE>;
     static cudaError_t attr = set_smem(fn, L::bytes);
     if (attr) return attr;
-    const int grid = occupancy_grid((const void*)fn, T, L::bytes, n, sms);
+    // a CTA for every node until the chip is full (node_chunk)
+    const int grid = occupancy_grid((const void*)fn, T, L::bytes, SPARSE ? n : (u64)n * T, sms);
     fn<<<grid, T, L::bytes, st>>>(lv, start, n, acc, ticket, max_rem);
     return cudaGetLastError();
 }
@@ -65,7 +66,7 @@ cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* of
     auto fn = k_expand<S, SL, T, Q>;
     static cudaError_t attr = set_smem(fn, L::bytes);
     if (attr) return attr;
-    const int grid = occupancy_grid((const void*)fn, T, L::bytes, (u64)(b - a), sms);
+    const int grid = occupancy_grid((const void*)fn, T, L::bytes, (u64)(b - a) * T, sms);
     fn<<<grid, T, L::bytes, st>>>(in, start, a, b, offs, out, ticket, nullptr);
     return cudaGetLastError();
 }
@@ -114,6 +115,26 @@ cudaError_t count_level_any(int side, const LevelView& lv, u32 start, u32 n, u32
 {
     return side ? count_level_t<1, SL>(lv, start, n, cnt, min_rem, st, sms)
                 : count_level_t<0, SL>(lv, start, n, cnt, min_rem, st, sms);
+}
+
+template <int S, class SL>
+cudaError_t count_plan_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap, PlanOut* plan,
+                         u32* done, const u32* err, cudaStream_t st)
+{
+    auto fn = k_count_plan<S, SL>;
+    constexpr int smem = table_smem_bytes<SL>();
+    static cudaError_t attr = set_smem(fn, smem);
+    if (attr) return attr;
+    fn<<<(n + 255) / 256, 256, smem, st>>>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err);
+    return cudaGetLastError();
+}
+
+template <class SL>
+cudaError_t count_plan_any(int side, const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
+                           PlanOut* plan, u32* done, const u32* err, cudaStream_t st)
+{
+    return side ? count_plan_t<1, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, st)
+                : count_plan_t<0, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, st);
 }
 
 inline int small_grid(u32 n, int T) { return (int)std::max<u32>(1, std::min<u32>((n + T - 1) / T, 8192)); }
@@ -171,6 +192,7 @@ cudaError_t playouts(const Pos& start, u64 seed, u32 n, int min_plies, int max_p
 #define PG_DEFINE_OPS(SLT, NAME, ENUM)                                                                   \
     const SliderOps g_ops_##NAME = {#NAME,          ENUM,                    upload_tables<SLT>,           \
                                     leaf_any<SLT>,  expand_any<SLT>,         count_level_any<SLT>,         \
+                                    count_plan_any<SLT>,                                                          \
                                     count_batch<SLT>, gen_moves_batch<SLT>,  gen_boards_batch<SLT>,        \
                                     make_batch,     playouts<SLT>};
 
