@@ -542,10 +542,17 @@ int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_gro
     u32* dctr = E.tickets + MAX_TICKETS - 4;  // white count, black count, min depth, max depth
     PG_CUDA(cudaMemsetAsync(dctr, 0, 4 * sizeof(u32), E.stream));
     PG_CUDA(cudaMemsetAsync(dctr + 2, 0xFF, sizeof(u32), E.stream));
-    k_partition_roots<<<std::max<u32>(1, std::min<u32>((n + 255) / 256, 4096)), 256, 0, E.stream>>>(
-        d_pos, d_depths, n, E.lv[0].v, dctr, d_groups);
+    const u32 pgrid = std::max<u32>(1, std::min<u32>((n + 255) / 256, 4096));
+    if (E.plan_mode == PLAN_NONE) {
+        k_partition_roots<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].v, dctr, d_groups);
+        E.st.launches++;
+    } else {
+        k_side_flags<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].cnt, dctr);
+        PG_TRY(launch_scan(E.lv[0].cnt, n, E.lv[0].offs));
+        k_place_roots<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].v, E.lv[0].offs, dctr, d_groups);
+        E.st.launches += 2;
+    }
     PG_CUDA(cudaGetLastError());
-    E.st.launches++;
     u32 nw, mind, maxd;
     if (capturing) {
         nw = E.rec_part[0];

@@ -44,6 +44,37 @@ static __global__ void k_partition_roots(const Pos* __restrict__ in, const unsig
     }
 }
 
+// The same partition in the order of the roots, for a launch sequence that is
+// recorded and replayed with the chunk boundaries of its recording (those name
+// nodes by index, so a replay has to make the same order): side flags, their
+// scan, the roots into place.
+static __global__ void k_side_flags(const Pos* __restrict__ in, const unsigned char* __restrict__ depths, u32 n,
+                                    u32* __restrict__ white, u32* counters /* as k_partition_roots */)
+{
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const u32 d = depths[i];
+        white[i] = st_side(in[i]) ? 0u : 1u;
+        atomicMin(&counters[2], d);
+        atomicMax(&counters[3], d);
+    }
+}
+static __global__ void k_place_roots(const Pos* __restrict__ in, const unsigned char* __restrict__ depths, u32 n,
+                                     LevelView lv, const u64* __restrict__ whites_before, u32* counters,
+                                     const u32* __restrict__ groups)
+{
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const Pos b = in[i];
+        const u32 w = (u32)whites_before[i], slot = st_side(b) ? n - 1 - (i - w) : w;
+        store_board(lv, slot, b);
+        lv.grp[slot] = groups ? groups[i] : i;
+        lv.rem[slot] = depths[i];
+        if (i == 0) {
+            counters[0] = (u32)whites_before[n];
+            counters[1] = n - (u32)whites_before[n];
+        }
+    }
+}
+
 constexpr int SCAN_T = 256;
 constexpr int SCAN_V = 8;
 constexpr int SCAN_TILE = SCAN_T * SCAN_V;

@@ -53,3 +53,24 @@ def test_leaf_collects_live_nodes_of_a_sparse_level(pg, orc, n):
     want = distinct[np.arange(half) % len(boards)]
     assert np.array_equal(got[0::2], want)
     assert np.array_equal(got[1::2], want[:n // 2])
+
+
+@pytest.mark.parametrize("n", [1, 257, 8191, 8192, 8193])
+def test_counts_scan_and_plan_of_small_levels(pg, orc, n):
+    """A first level of n white-to-move nodes, at the size from which counts,
+    scan and plan are separate launches, with one chunk and with several."""
+    boards = pg.random_playouts(43, 40000, 2, 60)
+    boards = boards[(boards["pawns"] >> np.uint64(63)) == 0][:n]
+    depths = np.full(n, 3, np.uint8)
+    depths[::5] = 2
+    want, _ = orc.perft_batch(boards, depths, os.cpu_count() or 1)
+    assert np.array_equal(pg.perft_batch(boards, depths, slider="ks"), want)
+    pg.shutdown()
+    try:
+        pg.init(hbm_budget_bytes=1 << 20)  # 65,536 nodes a level: several chunks
+        assert np.array_equal(pg.perft_batch(boards, depths, slider="ks"), want)
+        assert np.array_equal(pg.perft_batch(boards, depths, slider="ks", graph=True), want)
+        assert np.array_equal(pg.perft_batch(boards, depths, slider="ks", graph=True), want)
+    finally:
+        pg.shutdown()
+        pg.init()
