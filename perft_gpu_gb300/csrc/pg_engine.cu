@@ -264,12 +264,12 @@ static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int mi
     const bool capturing = E.plan_mode == PLAN_REPLAY;
     if (minrem <= lp) {
         cudaEvent_t* ev = nullptr;
-        if (!capturing) {
+        if (!capturing && E.timing) {
             PG_TRY(leaf_timer_pair(ev));
             cudaEventRecord(ev[0], E.stream);
         }
         PG_TRY(launch_leaf(leaf_variant(v, L), side, lb.v, start, n, acc));
-        if (!capturing) cudaEventRecord(ev[1], E.stream);
+        if (ev) cudaEventRecord(ev[1], E.stream);
     }
     if (maxrem <= lp) return PG_OK;
     const u64 cap_next = level_cap_max();
@@ -348,6 +348,8 @@ static int autotune_locked()
     if (E.tuned) return PG_OK;
     const auto t0 = std::chrono::steady_clock::now();
     const pg_stats saved = E.st;
+    const bool timing = E.timing;
+    E.timing = true;
     struct Cal {
         int depth;
         u32 n;
@@ -413,6 +415,7 @@ static int autotune_locked()
         }
     }
     cudaFree(buf);
+    E.timing = timing;
     if (rc != PG_OK) return rc;
     for (int d = 0; d < 3; d++) {
         E.tuned_slider[d] = E.tuned_slider[3];
@@ -452,16 +455,34 @@ Variant pick_variant(const pg_opts* o)
 
 static bool valid_board(const pg_board& b)
 {
-    const u64 inner = INNER;
-    const u64 pawns = b.pawns & inner;
-    const u64 occ = pawns | b.knights | b.bishop_queens | b.rook_queens | b.kings;
-    if (pawns & (b.knights | b.bishop_queens | b.rook_queens | b.kings)) return false;
-    if (b.knights & (b.bishop_queens | b.rook_queens | b.kings)) return false;
-    if ((b.bishop_queens | b.rook_queens) & b.kings) return false;
-    if (b.white & ~occ) return false;
-    if (__builtin_popcountll(b.kings & b.white) != 1) return false;
-    if (__builtin_popcountll(b.kings & ~b.white) != 1) return false;
-    return true;
+    return board_ok(b.white, b.pawns, b.knights, b.bishop_queens, b.rook_queens, b.kings);
+}
+
+// the first board or depth (null: boards only) that a call does not accept, as
+// its error
+static int check_roots_host(const pg_board* pos, const uint8_t* depths, u32 n)
+{
+    for (u32 i = 0; i < n; i++) {
+        if (!valid_board(pos[i])) { set_error("position %u is not a valid board", i); return PG_ERR_INVALID_POSITION; }
+        if (depths && depths[i] > 15) { set_error("depth %u of position %u out of range 0..15", depths[i], i); return PG_ERR_INVALID_ARGUMENT; }
+    }
+    return PG_OK;
+}
+
+// The same for many boards already copied to the device: checked there before
+// anything runs on them (a million boards took the host 2.5 ms); the host looks
+// for the first bad one only when there is one.
+static int check_roots_device(const Pos* d_pos, const unsigned char* d_depths, const pg_board* pos, const uint8_t* depths, u32 n)
+{
+    Engine& E = engine();
+    u32* bad = (u32*)E.aux;
+    u32* h = (u32*)(E.host_scratch + 176);  // pinned
+    PG_CUDA(cudaMemsetAsync(bad, 0, sizeof(u32), E.stream));
+    k_check_roots<<<std::min<u32>((n + 255) / 256, 2048), 256, 0, E.stream>>>(d_pos, d_depths, n, bad);
+    PG_CUDA(cudaGetLastError());
+    PG_CUDA(cudaMemcpyAsync(h, bad, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
+    PG_CUDA(cudaStreamSynchronize(E.stream));
+    return *h ? check_roots_host(pos, depths, n) : PG_OK;
 }
 
 static int check_opts(const pg_opts* o)
@@ -501,11 +522,11 @@ static int begin_call(const pg_opts* o)
 {
     Engine& E = engine();
     E.st = pg_stats{};
+    E.timing = o && o->stats;
     E.leaf_ev_used = 0;
     E.ticket_next = 0;
     PG_CUDA(cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream));
     PG_CUDA(cudaMemsetAsync(E.err, 0, sizeof(u32), E.stream));
-    (void)o;
     return PG_OK;
 }
 
@@ -531,17 +552,18 @@ static int end_call(const pg_opts* o)
 // perft of n roots; each root's count is added to acc[group] (group =
 // groups[i], or i when groups is null).  acc is zeroed first when zero_acc.
 int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_groups, u32 n, u64* acc, bool zero_acc,
-               const Variant& v)
+               const Variant& v, const RootInfo* known)
 {
     Engine& E = engine();
     const bool capturing = E.plan_mode == PLAN_REPLAY;
+    const bool timed = !capturing && E.timing;
     E.leaf_ev_used = 0;
     PG_TRY(ensure_level(0, n));
     if (zero_acc) PG_CUDA(cudaMemsetAsync(acc, 0, (u64)n * sizeof(u64), E.stream));
     u32* ctr = (u32*)(E.host_scratch + 64);  // pinned, 4 words
     u32* dctr = E.tickets + MAX_TICKETS - 4;  // white count, black count, min depth, max depth
     PG_CUDA(cudaMemsetAsync(dctr, 0, 4 * sizeof(u32), E.stream));
-    PG_CUDA(cudaMemsetAsync(dctr + 2, 0xFF, sizeof(u32), E.stream));
+    if (!known) PG_CUDA(cudaMemsetAsync(dctr + 2, 0xFF, sizeof(u32), E.stream));
     const u32 pgrid = std::max<u32>(1, std::min<u32>((n + 255) / 256, 4096));
     if (E.plan_mode == PLAN_NONE) {
         k_partition_roots<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].v, dctr, d_groups);
@@ -558,6 +580,10 @@ int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_gro
         nw = E.rec_part[0];
         mind = E.rec_part[2];
         maxd = E.rec_part[3];
+    } else if (known) {
+        nw = known->white;
+        mind = known->mind;
+        maxd = known->maxd;
     } else {
         PG_CUDA(cudaMemcpyAsync(ctr, dctr, 4 * sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
         PG_CUDA(cudaStreamSynchronize(E.stream));
@@ -570,10 +596,10 @@ int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_gro
         set_error("depth %u out of range 0..15", maxd);
         return PG_ERR_INVALID_ARGUMENT;
     }
-    if (!capturing) cudaEventRecord(E.ev0, E.stream);
+    if (timed) cudaEventRecord(E.ev0, E.stream);
     PG_TRY(run_range(v, 0, 0, nw, 0, (int)mind, (int)maxd, acc));
     PG_TRY(run_range(v, 0, nw, n - nw, 1, (int)mind, (int)maxd, acc));
-    if (!capturing) {
+    if (timed) {
         cudaEventRecord(E.ev1, E.stream);
         PG_CUDA(cudaEventSynchronize(E.ev1));
         float ms = 0;
@@ -825,12 +851,12 @@ int perft_core_persistent(const Pos* d_pos, const unsigned char* d_depths, const
     PG_CUDA(cudaMemsetAsync(E.persist_ctl, 0, sizeof(PersistCtl), E.stream));
     PG_CUDA(cudaMemsetAsync(&E.persist_ctl->part[2], 0xFF, sizeof(u32), E.stream));
     PG_CUDA(cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream));
-    const bool capturing = E.plan_mode == PLAN_REPLAY;
-    if (!capturing) cudaEventRecord(E.ev0, E.stream);
+    const bool timed = E.plan_mode != PLAN_REPLAY && E.timing;
+    if (timed) cudaEventRecord(E.ev0, E.stream);
     int grid = 0;
     PG_CUDA(persist_launch(A, E.stream, E.num_sms, &grid));
     E.st.launches++;
-    if (!capturing) {
+    if (timed) {
         cudaEventRecord(E.ev1, E.stream);
         PG_CUDA(cudaEventSynchronize(E.ev1));
         float ms = 0;
@@ -844,13 +870,13 @@ int perft_core_persistent(const Pos* d_pos, const unsigned char* d_depths, const
 // batch perft with device inputs; d_out must not alias the inputs; maxd the
 // batch's largest depth when the caller knows it (else -1)
 static int perft_batch_device_locked(const Pos* d_pos, const unsigned char* d_depths, u32 n, u64* d_out,
-                                     const pg_opts* o, int maxd = -1)
+                                     const pg_opts* o, int maxd = -1, const RootInfo* known = nullptr)
 {
     if (o && o->persistent) {
         if (maxd < 0) PG_TRY(device_max_depth(d_depths, n, &maxd));
         return perft_core_persistent(d_pos, d_depths, nullptr, n, d_out, true, maxd);
     }
-    return perft_core(d_pos, d_depths, nullptr, n, d_out, true, pick_variant(o));
+    return perft_core(d_pos, d_depths, nullptr, n, d_out, true, pick_variant(o), known);
 }
 
 // The positions `plies` plies below root (all of them, in generateMoves
@@ -1103,6 +1129,8 @@ static void release_engine(Engine& E)
     if (E.plan_dev) cudaFree(E.plan_dev);
     if (E.plan_host) cudaFreeHost(E.plan_host);
     if (E.host_scratch) cudaFreeHost(E.host_scratch);
+    if (E.host_io) cudaFreeHost(E.host_io);
+    E.host_io = nullptr;
     if (E.aux) cudaFree(E.aux);
     if (E.persist_plan) cudaFree(E.persist_plan);
     if (E.persist_ctl) cudaFree(E.persist_ctl);
@@ -1170,6 +1198,7 @@ static int init_locked(Engine& E, const pg_config* cfg)
     PG_CUDA(cudaMalloc(&E.plan_dev, sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.plan_host, sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.host_scratch, 4096));
+    PG_CUDA(cudaMallocHost(&E.host_io, HOST_IO_ROOTS * (48 + 1 + 8) + 64));
     PG_CUDA(cudaMalloc(&E.aux, 256));
     PG_CUDA(cudaDeviceSynchronize());
     E.ready = true;
@@ -1195,7 +1224,7 @@ int pg_shutdown(void)
     return PG_OK;
 }
 
-static int op_batch(int op, const pg_board* pos, u32 n, void* out, u32* nout, int slider)
+static int op_batch(int op, const pg_board* pos, u32 n, void* out, u32* nout, int slider, bool check = false)
 {
     Engine& E = engine();
     const u64 in_bytes = (u64)n * sizeof(Pos);
@@ -1207,6 +1236,7 @@ static int op_batch(int op, const pg_board* pos, u32 n, void* out, u32* nout, in
     void* d_out = s + in_bytes;
     u32* d_n = (u32*)(s + in_bytes + out_bytes);
     PG_CUDA(cudaMemcpyAsync(d_in, pos, in_bytes, cudaMemcpyHostToDevice, E.stream));
+    if (check) PG_TRY(check_roots_device(d_in, nullptr, pos, nullptr, n));
     const SliderOps& ops = ops_for(slider);
     if (op == 0) PG_CUDA(ops.count_batch(d_in, n, (u32*)d_out, E.stream));
     else if (op == 1) PG_CUDA(ops.gen_moves_batch(d_in, n, (u16*)d_out, d_n, E.stream));
@@ -1230,9 +1260,9 @@ int pg_count_moves_batch(const pg_board* pos, uint32_t n, uint32_t* out)
     std::lock_guard<std::mutex> lk(E.mu);
     PG_TRY(check_ready());
     if (n == 0) return PG_OK;
-    for (u32 i = 0; i < n; i++)
-        if (!valid_board(pos[i])) { set_error("position %u is not a valid board", i); return PG_ERR_INVALID_POSITION; }
-    return op_batch(0, pos, n, out, nullptr, slider_of(PG_SLIDER_AUTO));
+    const bool many = n > HOST_IO_ROOTS;
+    if (!many) PG_TRY(check_roots_host(pos, nullptr, n));
+    return op_batch(0, pos, n, out, nullptr, slider_of(PG_SLIDER_AUTO), many);
 }
 
 int pg_count_moves(const pg_board* pos, uint32_t* out) { return pg_count_moves_batch(pos, 1, out); }
@@ -1433,10 +1463,10 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     PG_TRY(check_ready());
     PG_TRY(check_opts(opts));
     if (n == 0) return PG_OK;
-    for (u32 i = 0; i < n; i++) {
-        if (!valid_board(pos[i])) { set_error("position %u is not a valid board", i); return PG_ERR_INVALID_POSITION; }
-        if (depths[i] > 15) { set_error("depth %u of position %u out of range 0..15", depths[i], i); return PG_ERR_INVALID_ARGUMENT; }
-    }
+    // a small call is checked on the host and staged in pinned memory: its copies
+    // are one each way and do not wait
+    const bool small = n <= HOST_IO_ROOTS;
+    if (small) PG_TRY(check_roots_host(pos, depths, n));
     const u64 pb = (u64)n * 48, db = ((u64)n + 15) & ~15ull, ob = (u64)n * 8;
     PG_TRY(ensure_stage(pb + db + ob + 64));
     unsigned char* s = (unsigned char*)E.stage;
@@ -1444,8 +1474,22 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     unsigned char* d_dep = s + pb;
     u64* d_out = (u64*)(s + pb + db);
     PG_TRY(begin_call(opts));
-    PG_CUDA(cudaMemcpyAsync(d_pos, pos, pb, cudaMemcpyHostToDevice, E.stream));
-    PG_CUDA(cudaMemcpyAsync(d_dep, depths, n, cudaMemcpyHostToDevice, E.stream));
+    RootInfo info{0, 15, 0};
+    if (small) {
+        memcpy(E.host_io, pos, pb);
+        memcpy(E.host_io + pb, depths, n);
+        for (u32 i = 0; i < n; i++) {
+            info.white += !(pos[i].pawns >> 63);
+            info.mind = std::min<u32>(info.mind, depths[i]);
+            info.maxd = std::max<u32>(info.maxd, depths[i]);
+        }
+        PG_CUDA(cudaMemcpyAsync(d_pos, E.host_io, pb + n, cudaMemcpyHostToDevice, E.stream));
+    } else {
+        PG_CUDA(cudaMemcpyAsync(d_pos, pos, pb, cudaMemcpyHostToDevice, E.stream));
+        PG_CUDA(cudaMemcpyAsync(d_dep, depths, n, cudaMemcpyHostToDevice, E.stream));
+        PG_TRY(check_roots_device(d_pos, d_dep, pos, depths, n));
+        for (u32 i = 0; i < n; i++) info.maxd = std::max<u32>(info.maxd, depths[i]);
+    }
     if (opts && opts->use_tt) {
         PG_TRY(tt_perft_batch_device(d_pos, d_dep, n, d_out, opts));
     } else if (opts && opts->graph && opts->persistent) {
@@ -1453,12 +1497,12 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     } else if (opts && opts->graph) {
         PG_TRY(perft_batch_graph_locked(d_pos, d_dep, n, d_out, opts));
     } else {
-        int maxd = 0;
-        for (u32 i = 0; i < n; i++) maxd = std::max<int>(maxd, depths[i]);
-        PG_TRY(perft_batch_device_locked(d_pos, d_dep, n, d_out, opts, maxd));
+        PG_TRY(perft_batch_device_locked(d_pos, d_dep, n, d_out, opts, (int)info.maxd, small ? &info : nullptr));
     }
-    PG_CUDA(cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
+    unsigned char* h_out = small ? E.host_io + pb + db : (unsigned char*)out;
+    PG_CUDA(cudaMemcpyAsync(h_out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
     PG_TRY(end_call(nullptr));
+    if (small) memcpy(out, h_out, ob);
     u64 total = 0;
     for (u32 i = 0; i < n; i++) total += out[i];
     E.st.leaves = total;

@@ -18,6 +18,7 @@ constexpr int MAX_LEVELS = 16;
 constexpr u64 LEVEL_NODE_BYTES = 48 + 4 + 1 + 4 + 8;
 constexpr u32 MAX_CHUNKS = 2048;      // greedy chunks planned per expansion
 constexpr u32 PLAN_FUSED_MAX = 8192;  // nodes of a level whose counts, scan and plan are one launch
+constexpr u32 HOST_IO_ROOTS = 4096;   // largest host-array call staged in pinned memory and checked on the host
 constexpr u32 MAX_TICKETS = 1 << 16;  // dynamic-scheduling counters per call
 
 // device error bits (bounded waits and capacity guards set them; no trap)
@@ -145,6 +146,8 @@ struct Engine {
     void* stage = nullptr;         // staging for host-array calls
     u64 stage_cap = 0;
     u64* host_scratch = nullptr;   // pinned small scratch
+    unsigned char* host_io = nullptr;  // pinned inputs and counts of a small host-array call
+    bool timing = true;            // the call records its launches' times (it returns stats)
     u64* aux = nullptr;            // small device scratch (input checksum)
     PlanOut* persist_plan = nullptr;  // MAX_LEVELS chunk plans of a persistent launch
     PersistCtl* persist_ctl = nullptr;
@@ -193,8 +196,12 @@ int launch_scan(const u32* cnt, u32 n, u64* offs);
 u64 level_cap_max();
 int ensure_level(int L, u64 need);
 int ensure_stage(u64 bytes);
+// what the host knows of a call's roots: white to move, smallest and largest depth
+struct RootInfo {
+    u32 white, mind, maxd;
+};
 int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_groups, u32 n, u64* acc, bool zero_acc,
-               const Variant& v);
+               const Variant& v, const RootInfo* known = nullptr);
 int expand_frontier(const Pos& root, int plies, Pos* out, u32 cap, u32* n_out);
 int perft_core_persistent(const Pos* d_pos, const unsigned char* d_depths, const u32* d_groups, u32 n, u64* acc,
                           bool zero_acc, int maxd);

@@ -25,6 +25,27 @@ __device__ __forceinline__ void store_board(const LevelView& lv, u64 i, const Po
     lv.pl2[i] = make_ulonglong2(p.rq, p.k);
 }
 
+// the checks of a caller's board: one king a side, no square held twice, white's
+// pieces among the pieces
+__host__ __device__ __forceinline__ bool board_ok(u64 w, u64 p, u64 n, u64 bq, u64 rq, u64 k)
+{
+    const u64 pawns = p & INNER, sliders = bq | rq;
+    const u64 twice = (pawns & (n | sliders | k)) | (n & (sliders | k)) | (sliders & k);
+    const u64 kw = k & w, kb = k & ~w;
+    return !(twice | (w & ~(pawns | n | sliders | k))) && kw && !(kw & (kw - 1)) && kb && !(kb & (kb - 1));
+}
+
+// *bad = 1 when a board (or, with depths, its depth) is not one a call accepts
+static __global__ void k_check_roots(const Pos* __restrict__ in, const unsigned char* __restrict__ depths, u32 n, u32* bad)
+{
+    bool ok = true;
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const Pos b = in[i];
+        ok = ok && board_ok(b.w, b.p, b.n, b.bq, b.rq, b.k) && !(depths && depths[i] > 15);
+    }
+    if (!ok) *bad = 1;
+}
+
 // roots into level 0, white-to-move first, black-to-move from the end
 static __global__ void k_partition_roots(const Pos* __restrict__ in, const unsigned char* __restrict__ depths, u32 n,
                                   LevelView lv, u32* counters /* [0] white, [1] black, [2] min depth, [3] max depth */,

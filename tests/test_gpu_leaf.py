@@ -74,3 +74,28 @@ def test_counts_scan_and_plan_of_small_levels(pg, orc, n):
     finally:
         pg.shutdown()
         pg.init()
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 30000])
+@pytest.mark.parametrize("bad", ["board", "depth", "both"])
+def test_batches_report_the_first_bad_root(pg, n, bad):
+    """The host checks small batches, the device large ones: same answer."""
+    boards = pg.random_playouts(47, n, 0, 40)
+    depths = np.full(n, 1, np.uint8)
+    moves = pg.count_moves_batch(boards)
+    assert np.array_equal(pg.perft_batch(boards, depths), moves)
+    spoilt, deep = boards.copy(), depths.copy()
+    if bad != "depth":
+        spoilt["kings"][n - 2] = 0
+    if bad != "board":
+        deep[n - 3] = 16
+    for options in ({}, {"persistent": True}, {"use_tt": "dedup"}):
+        with pytest.raises(pg.PerftError) as e:
+            pg.perft_batch(spoilt, deep, **options)
+        assert e.value.status == (3 if bad == "board" else 2)
+        assert str(n - 2 if bad == "board" else n - 3) in str(e.value)
+    if bad == "board":
+        with pytest.raises(pg.PerftError) as e:
+            pg.count_moves_batch(spoilt)
+        assert e.value.status == 3 and str(n - 2) in str(e.value)
+    assert np.array_equal(pg.perft_batch(boards, depths), moves)
