@@ -200,7 +200,7 @@ LevelView from_node(const LevelView& lv, u64 k)
 template <int S>
 void launch_leaf_na(const LevelView& lv, u32 start, u32 n, u64* out, u32* ticket, cudaStream_t st, int sms)
 {
-    constexpr int T = 128, Q = T * 24;
+    constexpr int T = 128, Q = T * 16;
     using L = LeafSmem<SlKS, T, Q>;
     static_assert(L::bytes <= 48 * 1024, "dynamic shared memory above the default limit");
     auto fn = k_leaf<S, SlKS, T, Q, false>;

@@ -10,12 +10,15 @@ namespace pg {
 namespace {
 
 // shared-memory queue entries per CTA.  The leaf queues the moves that are not
-// counted in sets, about 10 a node: 24 per thread hold them in one window.
+// counted in sets, about 10 a node: 16 per thread hold them in one window on
+// most CTAs, and a CTA with more gathers another window from its columns.
+// (Every 16th position of the batched workload: 30.7 ms with 16, 30.8 with 20
+// to 32, 31.0 with 12: what the queue takes is missing in the L1.)
 // The expansion queues every move: 64 per thread hold the children of nodes
 // with ~50 moves.  The byte-lookup policy gives 158 KB of the CTA's shared
 // memory to its tables and keeps 8.
 template <class SL, int T> struct QcapFor {
-    static constexpr int leaf = SL::kId == 2 ? T * 8 : T * 24;
+    static constexpr int leaf = SL::kId == 2 ? T * 8 : T * 16;
     static constexpr int expand = SL::kId == 2 ? T * 8 : T * 64;
 };
 

@@ -39,7 +39,7 @@ namespace pg {
 constexpr u64 PERSIST_BARRIER_NS = 60ull * 1000 * 1000 * 1000;  // 60 s of global time per barrier
 constexpr int PERSIST_T = PERSIST_CTA;
 constexpr int PERSIST_Q = PERSIST_T * 64;                        // queue entries per CTA (as k_expand)
-constexpr int PERSIST_LEAF_Q = PERSIST_T * 24;                   // and in the leaf phase (as k_leaf)
+constexpr int PERSIST_LEAF_Q = PERSIST_T * 16;                   // and in the leaf phase (as k_leaf)
 constexpr int PERSIST_SCAN_V = 4;                                // counts per thread per scan tile
 constexpr int PERSIST_SCAN_TILE = PERSIST_T * PERSIST_SCAN_V;
 static_assert(PERSIST_SCAN_TILE == (int)PERSIST_SCAN_TILE_NODES, "scan tile known to the host");

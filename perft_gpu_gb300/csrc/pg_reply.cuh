@@ -68,20 +68,20 @@ struct Planes3 {
 // ray; at the other side's piece it ends on, what that piece leaving opens.
 // s: the sliders' attack fill along one direction (blockers included), x: the
 // same from the squares of `blockers` it ends on, own: the sliders' side (not a
-// target), sl: the sliders.  The run of targets is followed back one step at a
-// time, through empty squares only; the opened squares themselves hold nothing.
+// target), sl: the sliders.  Runs of targets go through empty squares only; the
+// opened squares themselves hold nothing.
 template <int SH, bool LEFT>
 __device__ __forceinline__ Planes3 targets_beyond(u64 s, u64 x, u64 empty, u64 own, u64 sl, u64 blockers)
 {
     const u64 through = (s | x) & empty, at = through | sl | (s & blockers), keep = ~(x & empty);
-    auto back = [](u64 y) { return LEFT ? (y >> SH) : (y << SH); };
-    const u64 r1 = back((s | x) & ~own) & at;
-    const u64 r2 = back(r1 & through) & at;
-    const u64 r3 = back(r2 & through) & at;
-    const u64 r4 = back(r3 & through) & at;
-    const u64 r5 = back(r4 & through) & at;
-    const u64 r6 = back(r5 & through) & at;
-    const u64 r7 = back(r6 & through) & at;
+    auto back = [](u64 y, int k) { return LEFT ? (y >> (k * SH)) : (y << (k * SH)); };
+    // r_k: a run of k or more targets; by doubling, a run of k from the k-th
+    // square of a run of j is one of j + k
+    const u64 r1 = back((s | x) & ~own, 1) & at, e1 = r1 & through;
+    const u64 r2 = r1 & back(e1, 1), e2 = r2 & through;
+    const u64 r3 = r2 & back(e1, 2), e3 = r3 & through;
+    const u64 r4 = r2 & back(e2, 2);
+    const u64 r5 = r4 & back(e1, 4), r6 = r4 & back(e2, 4), r7 = r4 & back(e3, 4);
     return Planes3{((r1 & ~r2) | (r3 & ~r4) | (r5 & ~r6) | r7) & keep, ((r2 & ~r4) | r6) & keep, r4 & keep};
 }
 
