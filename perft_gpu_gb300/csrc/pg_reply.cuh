@@ -325,13 +325,14 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         n0 += 3 * (popc(x1 & back_rank) + popc(xw & back_rank) + popc(xe & back_rank));
         if (path) n0 += can_castle_k<T>(b, occ, thr) + can_castle_q<T>(b, occ, thr);
     }
-    // promotion squares count four times: not plain; neither is a piece that
-    // blocks a double push
-    const u64 fronts = push1<T>(op) & mine;
+    // pieces of the mover that stand in front of an opposing pawn, and (open2) two
+    // squares in front of one that could step twice; promotion squares count four
+    // times: not plain
+    const u64 fronts = push1<T>(op) & mine, open2 = push1<T>(mid) & mine;
     {
         const u64 pr8 = (push1<T>(op) | cw | ce) & back_rank;
         no_t |= pr8;
-        no_f |= pr8 | (fronts & double_rank<T>()) | push1<T>(mid);
+        no_f |= pr8;
     }
 
     // w: per square the replies lost when a piece arrives, plus 2: on an empty
@@ -470,8 +471,10 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         const u64 near_f = king_f | cap_w<T>(u_once) | cap_e<T>(u_once);
         const u64 near_t = king_t | pawn_attackers_of<T>(u0);
         const u64 no = no_t | pawn_attackers_of<T>(king) | BACK_RANKS | (near_t & strict);
-        const u64 stay_x = no_f | (near_f & strict), stay = stay_x | fronts;
+        const u64 stay_x = no_f | (near_f & strict), stay = stay_x | fronts | open2;
         // the replies that leaving the squares of x gives, plus 2 a square
+        // the pushes a capturing pawn leaves open behind it
+        auto pushes = [&](u64 x) { return popc(x & (fronts | open2)) + popc(push1<T>(x & fronts & double_rank<T>()) & empty); };
         auto leave = [&](u64 x) { return popc(x & w0) + 2 * popc(x & w1) + 4 * popc(x & w2) + 8 * popc(x & w3); };
         {
             const u64 ok = one & ~no & ~push1<S>(stay | s0 | s1);
@@ -499,7 +502,7 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
             const u64 ok = xw & ~no & ~cap_w<S>(stay_x | (S ? s4 | s5 : s6 | s7));
             const u64 from = S ? ok << 9 : ok >> 7, by_king = ok & (near_t | cap_w<S>(near_f));
             reach(ok);
-            sum += popc(ok) * n0 + leave(from) + popc(from & ce) + popc(from & fronts);
+            sum += popc(ok) * n0 + leave(from) + popc(from & ce) + pushes(from);
             const u64 rest = xw & ~ok & ~BACK_RANKS;
             emit.sets(pawn_set<CW>(rest), pawn_set<CW>(by_king), pawn_entry<CW>(), 65u);
             put_promotions(emit, xw & BACK_RANKS, CW);
@@ -508,7 +511,7 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
             const u64 ok = xe & ~no & ~cap_e<S>(stay_x | (S ? s6 | s7 : s4 | s5));
             const u64 from = S ? ok << 7 : ok >> 9, by_king = ok & (near_t | cap_e<S>(near_f));
             reach(ok);
-            sum += popc(ok) * n0 + leave(from) + popc(from & cw) + popc(from & fronts);
+            sum += popc(ok) * n0 + leave(from) + popc(from & cw) + pushes(from);
             const u64 rest = xe & ~ok & ~BACK_RANKS;
             emit.sets(pawn_set<CE>(rest), pawn_set<CE>(by_king), pawn_entry<CE>(), 65u);
             put_promotions(emit, xe & BACK_RANKS, CE);
@@ -522,15 +525,19 @@ template <int S, class E> __device__ __forceinline__ u64 reply_sum(const Pos& b,
         const bool hi = q >= 32;
         const u32 sq = q & 31;
         auto at = [&](u64 x) { return ((hi ? (u32)(x >> 32) : (u32)x) >> sq) & 1u; };
-        const u64 pawn_att = __ldg(&g_pawn_checks[S][q]) & op, front = push1<S>(fronts & bit);
-        no |= no_t | full() | pawn_att | front;
+        // pawns that could capture it, the pawn it blocks and that pawn's second
+        // step, the pawn whose second step it blocks and that one's first: t there
+        // is not plain
+        const u64 pawn_att = __ldg(&g_pawn_checks[S][q]) & op, in_front = fronts & bit, front = push1<S>(in_front);
+        const u64 second = push1<T>(in_front & double_rank<T>()), back2 = push1<S>(open2 & bit);
+        no |= no_t | full() | pawn_att | front | second | back2 | push1<S>(back2);
         near |= king_t;
         if ((bit & king_f) | (att & u_once)) near = ~0ull;
         no |= near & strict;
         if (bit & no_f) no = ~0ull;
         const u64 plain = to & ~no, by_king = plain & near, rest = to & no;
         reach(plain);
-        sum += popc(plain) * (n0 + (front != 0) + at(w0) + 2 * at(w1) + 4 * at(w2) + 8 * at(w3));
+        sum += popc(plain) * (n0 + (front != 0) + ((second & empty) != 0) + (back2 != 0) + at(w0) + 2 * at(w1) + 4 * at(w2) + 8 * at(w3));
         emit.sets(rest, by_king, (u32)q | (pc << Q_PIECE_SHIFT), 64u);
     };
     const u64 sv = s0 | s1, sh = s2 | s3, sd = s4 | s5, sa = s6 | s7;
