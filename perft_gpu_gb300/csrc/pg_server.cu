@@ -43,10 +43,16 @@ namespace {
 
 constexpr int TASK_DEPTH = 5;               // remaining depth of one task
 constexpr u32 MAX_WAVE_TASKS = 1u << 16;
+// Target device time of one wave: a newcomer waits for the rest of the running
+// wave and for its own, and a wave costs about 0.2 ms of launches and of levels too
+// small for the device.  8.7e10 leaves with a small request joining after 5 ms, the
+// small one's latency and the deep one's time at 4 / 3 / 2.5 / 2 ms: 7.1 / 5.1 /
+// 4.0 / 3.2 ms and 32.1 / 32.7 / 33.0 / 33.6 ms; 64 mixed requests 11.0 / 11.3 /
+// 11.5 / 12.6 ms.
 #ifndef PG_WAVE_SECONDS
-#define PG_WAVE_SECONDS 0.004
+#define PG_WAVE_SECONDS 0.0025
 #endif
-constexpr double WAVE_SECONDS = PG_WAVE_SECONDS;  // target device time of one wave
+constexpr double WAVE_SECONDS = PG_WAVE_SECONDS;
 constexpr double MIN_WAVE_LEAVES = 1e9;     // floor of the timed wave budget
 constexpr double MAX_WAVE_LEAVES = 4e10;
 
