@@ -152,6 +152,26 @@ struct QWindow {
         kings += popc(by_king);
     }
 };
+// One node's sum of replies and its queued moves, out of line: the call fixes
+// which registers are live across the node phase, and the compiler spills a
+// quarter as much as with the sum inlined into the queue's loops (260 -> 80 bytes
+// a thread at 128 registers).  Board and results go in registers.  The batch
+// workload's leaf 30.5 -> 29.9 ms, one position at depth 7 30.7 -> 29.4 ms, the
+// persistent launch 32.7 -> 31.8 ms; the queued moves' count and king recount as
+// calls of their own are slower (30.9 and 30.7 ms: their results are few and their
+// boards live already).
+struct Replies {
+    u64 sum;
+    u32 made, kings, eps;
+};
+template <int S, int STRIDE, int CAP>
+__device__ __noinline__ Replies node_replies(u64 w, u64 p, u64 n, u64 bq, u64 rq, u64 k, u32* column, u32 tag)
+{
+    const Pos b{w, p, n, bq, rq, k};
+    QColumn<STRIDE, CAP> e{column, tag, 0u, 0u, 0u};
+    const u64 sum = reply_sum<S>(b, e);
+    return Replies{sum, e.made, e.kings, e.eps};
+}
 // one node's part of a queue window (rare: a CTA with more children than its
 // queue holds), out of line so that the leaf keeps one copy of reply_sum
 template <int S> __device__ __noinline__ void queue_window(const Pos& b, u32* q, u32 off, u32 lo, u32 hi, u32 tag)
