@@ -417,6 +417,8 @@ static int autotune_locked()
     cudaFree(buf);
     E.timing = timing;
     if (rc != PG_OK) return rc;
+    E.ticket_next = 0;  // the counters as it found them
+    PG_CUDA(cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream));
     for (int d = 0; d < 3; d++) {
         E.tuned_slider[d] = E.tuned_slider[3];
         E.tuned_T[d] = E.tuned_T[3];
@@ -525,16 +527,16 @@ static int begin_call(const pg_opts* o)
     E.timing = o && o->stats;
     E.leaf_ev_used = 0;
     E.ticket_next = 0;
-    PG_CUDA(cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream));
-    PG_CUDA(cudaMemsetAsync(E.err, 0, sizeof(u32), E.stream));
+    PG_CUDA(cudaMemsetAsync(E.tickets, 0, (MAX_TICKETS + 1) * sizeof(u32), E.stream));  // and the error bits
     return PG_OK;
 }
 
-static int end_call(const pg_opts* o)
+// delivered: the error bits are on their way to host_scratch (k_deliver)
+static int end_call(const pg_opts* o, bool delivered = false)
 {
     Engine& E = engine();
     u32 errv = 0;
-    PG_CUDA(cudaMemcpyAsync(E.host_scratch, E.err, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
+    if (!delivered) PG_CUDA(cudaMemcpyAsync(E.host_scratch, E.err, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
     PG_CUDA(cudaStreamSynchronize(E.stream));
     errv = (u32)E.host_scratch[0];
     if (errv & (ERR_PLAN_OVERFLOW | ERR_LEVEL_CAP)) {
@@ -559,16 +561,18 @@ int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_gro
     const bool timed = !capturing && E.timing;
     E.leaf_ev_used = 0;
     PG_TRY(ensure_level(0, n));
-    if (zero_acc) PG_CUDA(cudaMemsetAsync(acc, 0, (u64)n * sizeof(u64), E.stream));
     u32* ctr = (u32*)(E.host_scratch + 64);  // pinned, 4 words
     u32* dctr = E.tickets + MAX_TICKETS - 4;  // white count, black count, min depth, max depth
-    PG_CUDA(cudaMemsetAsync(dctr, 0, 4 * sizeof(u32), E.stream));
-    if (!known) PG_CUDA(cudaMemsetAsync(dctr + 2, 0xFF, sizeof(u32), E.stream));
+    if (!known) {  // else as the call's start left them
+        PG_CUDA(cudaMemsetAsync(dctr, 0, 4 * sizeof(u32), E.stream));
+        PG_CUDA(cudaMemsetAsync(dctr + 2, 0xFF, sizeof(u32), E.stream));
+    }
     const u32 pgrid = std::max<u32>(1, std::min<u32>((n + 255) / 256, 4096));
     if (E.plan_mode == PLAN_NONE) {
-        k_partition_roots<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].v, dctr, d_groups);
+        k_partition_roots<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].v, dctr, d_groups, zero_acc ? acc : nullptr);
         E.st.launches++;
     } else {
+        if (zero_acc) PG_CUDA(cudaMemsetAsync(acc, 0, (u64)n * sizeof(u64), E.stream));
         k_side_flags<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].cnt, dctr);
         PG_TRY(launch_scan(E.lv[0].cnt, n, E.lv[0].offs));
         k_place_roots<<<pgrid, 256, 0, E.stream>>>(d_pos, d_depths, n, E.lv[0].v, E.lv[0].offs, dctr, d_groups);
@@ -1125,7 +1129,6 @@ static void release_engine(Engine& E)
     if (E.scan_status) cudaFree(E.scan_status);
     if (E.stage) cudaFree(E.stage);
     if (E.tickets) cudaFree(E.tickets);
-    if (E.err) cudaFree(E.err);
     if (E.plan_dev) cudaFree(E.plan_dev);
     if (E.plan_host) cudaFreeHost(E.plan_host);
     if (E.host_scratch) cudaFreeHost(E.host_scratch);
@@ -1193,8 +1196,8 @@ static int init_locked(Engine& E, const pg_config* cfg)
     PG_CUDA(g_ops_fancy.upload(*tabs));
     PG_CUDA(g_ops_byte.upload(*tabs));
     PG_CUDA(g_ops_hybrid.upload(*tabs));
-    PG_CUDA(cudaMalloc(&E.tickets, MAX_TICKETS * sizeof(u32)));
-    PG_CUDA(cudaMalloc(&E.err, 16));
+    PG_CUDA(cudaMalloc(&E.tickets, (MAX_TICKETS + 4) * sizeof(u32)));
+    E.err = E.tickets + MAX_TICKETS;
     PG_CUDA(cudaMalloc(&E.plan_dev, sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.plan_host, sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.host_scratch, 4096));
@@ -1463,9 +1466,10 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     PG_TRY(check_ready());
     PG_TRY(check_opts(opts));
     if (n == 0) return PG_OK;
-    // a small call is checked on the host and staged in pinned memory: its copies
-    // are one each way and do not wait
+    // a small call is checked on the host and staged in pinned memory, which the
+    // root partition reads and k_deliver writes: no copies of its own
     const bool small = n <= HOST_IO_ROOTS;
+    const bool in_place = small && !(opts && (opts->use_tt || opts->graph));
     if (small) PG_TRY(check_roots_host(pos, depths, n));
     const u64 pb = (u64)n * 48, db = ((u64)n + 15) & ~15ull, ob = (u64)n * 8;
     PG_TRY(ensure_stage(pb + db + ob + 64));
@@ -1483,7 +1487,12 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
             info.mind = std::min<u32>(info.mind, depths[i]);
             info.maxd = std::max<u32>(info.maxd, depths[i]);
         }
-        PG_CUDA(cudaMemcpyAsync(d_pos, E.host_io, pb + n, cudaMemcpyHostToDevice, E.stream));
+        if (in_place) {
+            d_pos = (Pos*)E.host_io;
+            d_dep = E.host_io + pb;
+        } else {
+            PG_CUDA(cudaMemcpyAsync(d_pos, E.host_io, pb + n, cudaMemcpyHostToDevice, E.stream));
+        }
     } else {
         PG_CUDA(cudaMemcpyAsync(d_pos, pos, pb, cudaMemcpyHostToDevice, E.stream));
         PG_CUDA(cudaMemcpyAsync(d_dep, depths, n, cudaMemcpyHostToDevice, E.stream));
@@ -1499,10 +1508,16 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     } else {
         PG_TRY(perft_batch_device_locked(d_pos, d_dep, n, d_out, opts, (int)info.maxd, small ? &info : nullptr));
     }
-    unsigned char* h_out = small ? E.host_io + pb + db : (unsigned char*)out;
-    PG_CUDA(cudaMemcpyAsync(h_out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
-    PG_TRY(end_call(nullptr));
-    if (small) memcpy(out, h_out, ob);
+    if (small) {
+        u64* h_out = (u64*)(E.host_io + pb + db);
+        k_deliver<<<(n + 255) / 256, 256, 0, E.stream>>>(d_out, n, h_out, E.err, (u32*)E.host_scratch);
+        PG_CUDA(cudaGetLastError());
+        PG_TRY(end_call(nullptr, true));
+        memcpy(out, h_out, ob);
+    } else {
+        PG_CUDA(cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
+        PG_TRY(end_call(nullptr));
+    }
     u64 total = 0;
     for (u32 i = 0; i < n; i++) total += out[i];
     E.st.leaves = total;

@@ -138,7 +138,7 @@ struct Engine {
     u64 scan_status_cap = 0;
     u32* tickets = nullptr;  // MAX_TICKETS counters, zeroed per call
     u32 ticket_next = 0;
-    u32* err = nullptr;
+    u32* err = nullptr;      // error bits, the word behind the counters (cleared with them)
     PlanOut* plan_dev = nullptr;
     PlanOut* plan_host = nullptr;  // pinned
     u64* acc = nullptr;            // per-group counters

@@ -49,7 +49,8 @@ static __global__ void k_check_roots(const Pos* __restrict__ in, const unsigned 
 // roots into level 0, white-to-move first, black-to-move from the end
 static __global__ void k_partition_roots(const Pos* __restrict__ in, const unsigned char* __restrict__ depths, u32 n,
                                   LevelView lv, u32* counters /* [0] white, [1] black, [2] min depth, [3] max depth */,
-                                  const u32* __restrict__ groups = nullptr /* group id per root; null = index */)
+                                  const u32* __restrict__ groups = nullptr /* group id per root; null = index */,
+                                  u64* zero = nullptr /* counts to clear, one a root */)
 {
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const Pos b = in[i];
@@ -60,6 +61,7 @@ static __global__ void k_partition_roots(const Pos* __restrict__ in, const unsig
         store_board(lv, slot, b);
         lv.grp[slot] = groups ? groups[i] : i;
         lv.rem[slot] = (unsigned char)d;
+        if (zero) zero[i] = 0;
         atomicMin(&counters[2], d);
         atomicMax(&counters[3], d);
     }
@@ -94,6 +96,14 @@ static __global__ void k_place_roots(const Pos* __restrict__ in, const unsigned 
             counters[1] = n - (u32)whites_before[n];
         }
     }
+}
+
+// the counts and the error bits of a small call into pinned host memory
+static __global__ void k_deliver(const u64* __restrict__ counts, u32 n, u64* __restrict__ out, const u32* __restrict__ err,
+                                 u32* __restrict__ err_out)
+{
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = counts[i];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;
 }
 
 constexpr int SCAN_T = 256;

@@ -22,13 +22,18 @@ template <class SL, int T> struct QcapFor {
     static constexpr int expand = SL::kId == 2 ? T * 8 : T * 64;
 };
 
-inline int occupancy_grid(const void* fn, int T, int smem, u64 items, int num_sms)
+// CTAs of a kernel an SM holds (each launch wrapper asks once)
+inline int resident_ctas(const void* fn, int T, int smem)
 {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, smem) != cudaSuccess || per_sm < 1) {
         cudaGetLastError();
         per_sm = 1;
     }
+    return per_sm;
+}
+inline int full_grid(int per_sm, int T, u64 items, int num_sms)
+{
     const u64 want = std::max<u64>(1, (items + T - 1) / T);
     return (int)std::min<u64>(want, (u64)per_sm * (u64)num_sms);
 }
@@ -55,7 +60,8 @@ cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket,
     static cudaError_t attr = set_smem(fn, L::bytes);
     if (attr) return attr;
     // a CTA for every node until the chip is full (node_chunk)
-    const int grid = occupancy_grid((const void*)fn, T, L::bytes, SPARSE ? n : (u64)n * T, sms);
+    static const int per_sm = resident_ctas((const void*)fn, T, L::bytes);
+    const int grid = full_grid(per_sm, T, SPARSE ? n : (u64)n * T, sms);
     fn<<<grid, T, L::bytes, st>>>(lv, start, n, acc, ticket, max_rem);
     return cudaGetLastError();
 }
@@ -69,7 +75,8 @@ cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* of
     auto fn = k_expand<S, SL, T, Q>;
     static cudaError_t attr = set_smem(fn, L::bytes);
     if (attr) return attr;
-    const int grid = occupancy_grid((const void*)fn, T, L::bytes, (u64)(b - a) * T, sms);
+    static const int per_sm = resident_ctas((const void*)fn, T, L::bytes);
+    const int grid = full_grid(per_sm, T, (u64)(b - a) * T, sms);
     fn<<<grid, T, L::bytes, st>>>(in, start, a, b, offs, out, ticket, nullptr);
     return cudaGetLastError();
 }
@@ -107,7 +114,8 @@ cudaError_t count_level_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 m
     constexpr int smem = table_smem_bytes<SL>();
     static cudaError_t attr = set_smem(fn, smem);
     if (attr) return attr;
-    const int grid = occupancy_grid((const void*)fn, 256, smem, n, sms);
+    static const int per_sm = resident_ctas((const void*)fn, 256, smem);
+    const int grid = full_grid(per_sm, 256, n, sms);
     fn<<<grid, 256, smem, st>>>(lv, start, n, cnt, min_rem);
     return cudaGetLastError();
 }

@@ -99,3 +99,13 @@ def test_batches_report_the_first_bad_root(pg, n, bad):
             pg.count_moves_batch(spoilt)
         assert e.value.status == 3 and str(n - 2) in str(e.value)
     assert np.array_equal(pg.perft_batch(boards, depths), moves)
+
+
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 4095, 4096, 4097])
+def test_small_calls_read_and_write_pinned_memory(pg, orc, n):
+    """Calls of up to 4,096 roots leave their boards and find their counts in
+    pinned memory: two calls with different roots, the counts cleared between."""
+    for seed, persistent in ((53, False), (59, False), (61, True)):
+        boards, depths = pg.random_playouts(seed, n, 0, 60, 1, 0, 2, with_depths=True)
+        want, _ = orc.perft_batch(boards, depths, os.cpu_count() or 1)
+        assert np.array_equal(pg.perft_batch(boards, depths, persistent=persistent), want)
