@@ -75,7 +75,7 @@ u32* next_ticket()
     }
 
 static constexpr u32 LEAF_SPARSE_MIN = 1u << 19;
-int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u64* acc, bool sparse)
+int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u64* acc, bool sparse, const u32* n_dev)
 {
     Engine& E = engine();
     // Collecting the live nodes of a level (k_leaf) pays once every one of the
@@ -84,7 +84,8 @@ int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 
     // depths) took 465 us against 328 us, since 1,024 nodes went to one CTA
     sparse = sparse && n >= LEAF_SPARSE_MIN;
     PG_TICKET(tk);
-    PG_CUDA(ops_for(v.slider).leaf(side, v.T, lv, start, n, acc, tk, (u32)v.leaf_plies, sparse, E.stream, E.num_sms));
+    PG_CUDA(ops_for(v.slider).leaf(side, v.T, lv, start, n, acc, tk, (u32)v.leaf_plies, sparse, n_dev, E.stream,
+                                   E.num_sms));
     E.st.launches++;
     E.st.leaf_kernel_launches++;
     E.st.leaf_parent_nodes += n;
@@ -92,11 +93,11 @@ int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 
 }
 
 int launch_expand(const Variant& v, int side, const LevelView& in, u32 start, u32 a, u32 b, const u64* offs,
-                         const LevelView& out)
+                         const LevelView& out, Ahead ahead)
 {
     Engine& E = engine();
     PG_TICKET(tk);
-    PG_CUDA(ops_for(v.slider).expand(side, v.T, in, start, a, b, offs, out, tk, E.stream, E.num_sms));
+    PG_CUDA(ops_for(v.slider).expand(side, v.T, in, start, a, b, offs, out, tk, ahead, E.stream, E.num_sms));
     E.st.launches++;
     return PG_OK;
 }
@@ -254,6 +255,9 @@ static int leaf_timer_pair(cudaEvent_t*& pair)
     return PG_OK;
 }
 
+static int run_children(const Variant& v, int L, u32 start, u32 n, int side, int minrem, int maxrem, u64* acc,
+                        const u32* n_dev);
+
 static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int minrem, int maxrem, u64* acc)
 {
     Engine& E = engine();
@@ -272,12 +276,24 @@ static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int mi
         if (ev) cudaEventRecord(ev[1], E.stream);
     }
     if (maxrem <= lp) return PG_OK;
+    return run_children(v, L, start, n, side, minrem, maxrem, acc, nullptr);
+}
+
+// The same without the level's own leaf: counts, plan, and each chunk's subtree.
+// n_dev: the level was launched ahead (run_ahead), n bounds its size and the
+// words before it tell whether all went well.
+static int run_children(const Variant& v, int L, u32 start, u32 n, int side, int minrem, int maxrem, u64* acc, const u32* n_dev)
+{
+    Engine& E = engine();
+    LevelBuf& lb = E.lv[L];
+    const int lp = v.leaf_plies;
+    const bool capturing = E.plan_mode == PLAN_REPLAY;
     const u64 cap_next = level_cap_max();
-    const bool fused = n <= PLAN_FUSED_MAX;
+    const bool fused = n <= PLAN_FUSED_MAX || n_dev;
     if (fused) {
         PG_TICKET(done);
         PG_CUDA(ops_for(v.slider).count_plan(side, lb.v, start, n, lb.cnt, (u32)lp + 1, lb.offs, cap_next, E.plan_host, done,
-                                             E.err, E.stream));
+                                             E.err, Ahead{n_dev, nullptr}, E.stream));
         E.st.launches++;
     } else {
         PG_TRY(launch_count(v, side, lb.v, start, n, lb.cnt));
@@ -300,6 +316,7 @@ static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int mi
         if (fused) {
             PG_CUDA(cudaStreamSynchronize(E.stream));
             errv = plan.pad;
+            if (n_dev) n = plan.bnd[1];
         }
         if (!fused || (plan.nchunks == 0 && !errv)) {
             k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_dev, E.err);
@@ -334,6 +351,54 @@ static int run_range(const Variant& v, int L, u32 start, u32 n, int side, int mi
         PG_TRY(run_range(v, L + 1, 0, (u32)children, 1 - side, cminrem, cmaxrem, acc));
     }
     return PG_OK;
+}
+
+// run_range for a few roots, without waiting for each level's size: counts,
+// expansions and leaves of the first levels are launched one behind the other
+// with bounds for their sizes, and read the sizes from device words.  The host
+// waits once the next level's bound is over the smallest level buffer, or only
+// at the end of the call.  A level whose children do not fit all the same (more
+// than AHEAD_MOVES a node, on boards of no game) stops the sequence on the
+// device; ahead_failed() tells afterwards, and the caller runs the whole call
+// level by level.  One position at depth 3 / 4 / 5: 66 / 93 / 126 us waiting at
+// each level, 60 / 81 / 114 us so.
+static int run_ahead(const Variant& v, u32 start, u32 n, int side0, int minrem, int maxrem, u64* acc)
+{
+    Engine& E = engine();
+    if (n == 0) return PG_OK;
+    const int lp = v.leaf_plies;
+    const u32* n_dev = nullptr;
+    int side = side0;
+    for (int L = 0;; L++) {
+        LevelBuf& lb = E.lv[L];
+        if (minrem <= lp) PG_TRY(launch_leaf(leaf_variant(v, L), side, lb.v, start, n, acc, false, n_dev));
+        if (maxrem <= lp) return PG_OK;
+        if ((u64)n * AHEAD_MOVES > AHEAD_NODES || E.ahead_plans == AHEAD_PLANS)
+            return run_children(v, L, start, n, side, minrem, maxrem, acc, n_dev);
+        PG_TRY(ensure_level(L + 1, n * AHEAD_MOVES));
+        const Ahead ahead{n_dev, E.ahead_n + E.ahead_plans};
+        PG_TICKET(done);
+        PG_CUDA(ops_for(v.slider).count_plan(side, lb.v, start, n, lb.cnt, (u32)lp + 1, lb.offs, E.lv[L + 1].cap,
+                                             E.plan_host + 1 + E.ahead_plans, done, E.err, ahead, E.stream));
+        E.st.launches++;
+        PG_TRY(launch_expand(v, side, lb.v, start, 0, n, lb.offs, E.lv[L + 1].v, ahead));
+        E.ahead_plans++;
+        n_dev = ahead.children;
+        n *= AHEAD_MOVES;
+        start = 0;
+        side = 1 - side;
+        minrem = std::max(minrem, lp + 1) - 1;
+        maxrem--;
+    }
+}
+
+// after the stream was waited for: whether a level launched ahead did not fit
+static bool ahead_failed()
+{
+    Engine& E = engine();
+    for (int k = 0; k < E.ahead_plans; k++)
+        if (E.plan_host[1 + k].nchunks == 0) return true;
+    return false;
 }
 
 // The autotuner: per root depth 3..6, a seeded calibration batch is timed
@@ -527,6 +592,7 @@ static int begin_call(const pg_opts* o)
     E.timing = o && o->stats;
     E.leaf_ev_used = 0;
     E.ticket_next = 0;
+    E.ahead_plans = 0;
     PG_CUDA(cudaMemsetAsync(E.tickets, 0, (MAX_TICKETS + 1) * sizeof(u32), E.stream));  // and the error bits
     return PG_OK;
 }
@@ -601,8 +667,12 @@ int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_gro
         return PG_ERR_INVALID_ARGUMENT;
     }
     if (timed) cudaEventRecord(E.ev0, E.stream);
-    PG_TRY(run_range(v, 0, 0, nw, 0, (int)mind, (int)maxd, acc));
-    PG_TRY(run_range(v, 0, nw, n - nw, 1, (int)mind, (int)maxd, acc));
+    // stats want each launch's nodes: level by level then
+    const bool ahead = known && known->ahead && E.plan_mode == PLAN_NONE && !E.timing;
+    E.ahead_plans = 0;
+    PG_TRY((ahead ? run_ahead(v, 0, nw, 0, (int)mind, (int)maxd, acc) : run_range(v, 0, 0, nw, 0, (int)mind, (int)maxd, acc)));
+    PG_TRY((ahead ? run_ahead(v, nw, n - nw, 1, (int)mind, (int)maxd, acc)
+                  : run_range(v, 0, nw, n - nw, 1, (int)mind, (int)maxd, acc)));
     if (timed) {
         cudaEventRecord(E.ev1, E.stream);
         PG_CUDA(cudaEventSynchronize(E.ev1));
@@ -1150,6 +1220,7 @@ static void release_engine(Engine& E)
     E.stream = nullptr;
     E.tickets = nullptr;
     E.err = nullptr;
+    E.ahead_n = nullptr;
     E.plan_dev = nullptr;
     E.plan_host = nullptr;
     E.host_scratch = nullptr;
@@ -1196,10 +1267,11 @@ static int init_locked(Engine& E, const pg_config* cfg)
     PG_CUDA(g_ops_fancy.upload(*tabs));
     PG_CUDA(g_ops_byte.upload(*tabs));
     PG_CUDA(g_ops_hybrid.upload(*tabs));
-    PG_CUDA(cudaMalloc(&E.tickets, (MAX_TICKETS + 4) * sizeof(u32)));
+    PG_CUDA(cudaMalloc(&E.tickets, (MAX_TICKETS + 4 + AHEAD_PLANS) * sizeof(u32)));
     E.err = E.tickets + MAX_TICKETS;
+    E.ahead_n = E.err + 4;
     PG_CUDA(cudaMalloc(&E.plan_dev, sizeof(PlanOut)));
-    PG_CUDA(cudaMallocHost(&E.plan_host, sizeof(PlanOut)));
+    PG_CUDA(cudaMallocHost(&E.plan_host, (1 + AHEAD_PLANS) * sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.host_scratch, 4096));
     PG_CUDA(cudaMallocHost(&E.host_io, HOST_IO_ROOTS * (48 + 1 + 8) + 64));
     PG_CUDA(cudaMalloc(&E.aux, 256));
@@ -1478,7 +1550,7 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     unsigned char* d_dep = s + pb;
     u64* d_out = (u64*)(s + pb + db);
     PG_TRY(begin_call(opts));
-    RootInfo info{0, 15, 0};
+    RootInfo info{0, 15, 0, true};
     if (small) {
         memcpy(E.host_io, pos, pb);
         memcpy(E.host_io + pb, depths, n);
@@ -1513,6 +1585,13 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
         k_deliver<<<(n + 255) / 256, 256, 0, E.stream>>>(d_out, n, h_out, E.err, (u32*)E.host_scratch);
         PG_CUDA(cudaGetLastError());
         PG_TRY(end_call(nullptr, true));
+        if (ahead_failed()) {  // once more, waiting for every level's size
+            info.ahead = false;
+            PG_TRY(begin_call(opts));
+            PG_TRY(perft_batch_device_locked(d_pos, d_dep, n, d_out, opts, (int)info.maxd, &info));
+            PG_CUDA(cudaMemcpyAsync(h_out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
+            PG_TRY(end_call(nullptr));
+        }
         memcpy(out, h_out, ob);
     } else {
         PG_CUDA(cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));

@@ -18,6 +18,11 @@ constexpr int MAX_LEVELS = 16;
 constexpr u64 LEVEL_NODE_BYTES = 48 + 4 + 1 + 4 + 8;
 constexpr u32 MAX_CHUNKS = 2048;      // greedy chunks planned per expansion
 constexpr u32 PLAN_FUSED_MAX = 8192;  // nodes of a level whose counts, scan and plan are one launch
+// Levels launched before the host knows their sizes (run_ahead): while AHEAD_MOVES
+// children a node, the most a position of a game has, fit the smallest level buffer
+constexpr u32 AHEAD_MOVES = 218;
+constexpr u32 AHEAD_NODES = 1u << 16;
+constexpr int AHEAD_PLANS = 4;  // two levels for each side of the roots (1 x 218 x 218 is under AHEAD_NODES)
 constexpr u32 HOST_IO_ROOTS = 4096;   // largest host-array call staged in pinned memory and checked on the host
 constexpr u32 MAX_TICKETS = 1 << 16;  // dynamic-scheduling counters per call
 
@@ -40,6 +45,12 @@ struct LevelView {
     ulonglong2* pl2;  // (rook_queens, kings)
     u32* grp;
     unsigned char* rem;
+};
+
+// device words of a level launched before the host knows it (run_ahead)
+struct Ahead {
+    const u32* nodes = nullptr;  // the level's nodes (null: the launch's argument)
+    u32* children = nullptr;     // its children, 0 when they do not fit the next level
 };
 
 struct LevelBuf {
@@ -140,7 +151,9 @@ struct Engine {
     u32 ticket_next = 0;
     u32* err = nullptr;      // error bits, the word behind the counters (cleared with them)
     PlanOut* plan_dev = nullptr;
-    PlanOut* plan_host = nullptr;  // pinned
+    PlanOut* plan_host = nullptr;  // pinned: the plan waited for, then one for each level launched ahead
+    u32* ahead_n = nullptr;        // nodes of the levels launched ahead
+    int ahead_plans = 0;           // how many the call has launched
     u64* acc = nullptr;            // per-group counters
     u64 acc_cap = 0;
     void* stage = nullptr;         // staging for host-array calls
@@ -188,17 +201,21 @@ struct Variant {
 Variant pick_variant(const pg_opts* o);
 u32* next_ticket();
 // sparse: many nodes of the range are dead
-int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u64* acc, bool sparse = false);
+// n_dev: the number of nodes on the device, n a bound
+int launch_leaf(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u64* acc, bool sparse = false,
+                const u32* n_dev = nullptr);
 int launch_expand(const Variant& v, int side, const LevelView& in, u32 start, u32 a, u32 b, const u64* offs,
-                  const LevelView& out);
+                  const LevelView& out, Ahead ahead = Ahead{});
 int launch_count(const Variant& v, int side, const LevelView& lv, u32 start, u32 n, u32* cnt);
 int launch_scan(const u32* cnt, u32 n, u64* offs);
 u64 level_cap_max();
 int ensure_level(int L, u64 need);
 int ensure_stage(u64 bytes);
-// what the host knows of a call's roots: white to move, smallest and largest depth
+// what the host knows of a call's roots: white to move, smallest and largest
+// depth; ahead: first levels may be launched ahead, the caller asks ahead_failed()
 struct RootInfo {
     u32 white, mind, maxd;
+    bool ahead;
 };
 int perft_core(const Pos* d_pos, const unsigned char* d_depths, const u32* d_groups, u32 n, u64* acc, bool zero_acc,
                const Variant& v, const RootInfo* known = nullptr);

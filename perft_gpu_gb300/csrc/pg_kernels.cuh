@@ -324,11 +324,15 @@ __global__ void k_count_level(LevelView lv, u32 start, u32 n, u32* __restrict__ 
 // PLAN_FUSED_MAX) in one launch: the last CTA to finish its counts scans them
 // all.  The plan goes straight to pinned host memory (nchunks 0: the children do
 // not fit one chunk of `cap`, k_plan has to split them; pad: the error bits).
+// ahead: the level's size (null: n) and where its children's number goes for a
+// launch sequence that does not return to the host between levels; 0 there when
+// they do not fit, so that the launches behind do nothing.
 template <int S, class SL>
 __global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
-                                                    PlanOut* plan, u32* done, const u32* err)
+                                                    PlanOut* plan, u32* done, const u32* err, Ahead ahead)
 {
     stage_tables<SL>();
+    if (ahead.nodes) n = *ahead.nodes;
     count_level_body<S, SL>(lv, start, n, cnt, min_rem);
     constexpr int T = 256;
     __shared__ u32 s_done;
@@ -363,6 +367,7 @@ __global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32
     if (tid == 0) {
         offs[n] = total;
         plan->nchunks = total <= cap ? 1u : 0u;
+        if (ahead.children) *ahead.children = total <= cap ? (u32)total : 0u;
         plan->pad = *err;
         plan->total = total;
         plan->bnd[0] = 0;
@@ -418,7 +423,8 @@ template <int T> constexpr int min_blocks() { return (PG_LEAF_MIN_WARPS * 32 + T
 // than calling the inlined function).  LV is LevelView or any type with the
 // same grp[] / rem[] subscripts and a load_board overload.
 template <int S, class SL, int T, int QCAP, bool SPARSE, class LV>
-__device__ __forceinline__ void leaf_body(LV lv, u32 start, u32 n, u64* __restrict__ acc, u32* ticket, u32 max_rem)
+__device__ __forceinline__ void leaf_body(LV lv, u32 start, u32 n, u64* __restrict__ acc, u32* ticket, u32 max_rem,
+                                          const u32* n_dev)
 {
     extern __shared__ __align__(16) unsigned char pg_dyn_smem[];
 #include "pg_leaf_body.inc"
@@ -426,7 +432,7 @@ __device__ __forceinline__ void leaf_body(LV lv, u32 start, u32 n, u64* __restri
 
 template <int S, class SL, int T, int QCAP, bool SPARSE>
 __global__ void __launch_bounds__(T, min_blocks<T>()) k_leaf(LevelView lv, u32 start, u32 n, u64* __restrict__ acc, u32* ticket,
-                                                            u32 max_rem)
+                                                            u32 max_rem, const u32* __restrict__ n_dev)
 {
     extern __shared__ __align__(16) unsigned char pg_dyn_smem[];
     stage_tables<SL>();
@@ -506,9 +512,14 @@ __device__ __forceinline__ void expand_body(const LevelView& in, u32 start, u32 
 
 template <int S, class SL, int T, int QCAP>
 __global__ void __launch_bounds__(T, min_blocks<T>()) k_expand(LevelView in, u32 start, u32 a, u32 b, const u64* __restrict__ offs,
-                                              LevelView out, u32* ticket, u32* __restrict__ parent_out = nullptr)
+                                              LevelView out, u32* ticket, u32* __restrict__ parent_out = nullptr,
+                                              Ahead ahead = Ahead{})
 {
     stage_tables<SL>();
+    if (ahead.children) {
+        if (*ahead.children == 0) return;  // none, or more than `out` holds
+        if (ahead.nodes) b = *ahead.nodes;
+    }
     expand_body<S, SL, T, QCAP>(in, start, a, b, offs, out, ticket, parent_out);
 }
 

@@ -204,7 +204,7 @@ void launch_leaf_na(const LevelView& lv, u32 start, u32 n, u64* out, u32* ticket
     using L = LeafSmem<SlKS, T, Q>;
     static_assert(L::bytes <= 48 * 1024, "dynamic shared memory above the default limit");
     auto fn = k_leaf<S, SlKS, T, Q, false>;
-    fn<<<grid_of((const void*)fn, T, L::bytes, (u64)n * T, sms), T, L::bytes, st>>>(lv, start, n, out, ticket, 2u);
+    fn<<<grid_of((const void*)fn, T, L::bytes, (u64)n * T, sms), T, L::bytes, st>>>(lv, start, n, out, ticket, 2u, nullptr);
 }
 
 template <int S>
@@ -215,7 +215,7 @@ void launch_expand_na(const LevelView& in, u32 start, u32 a, u32 b, const u64* o
     using L = BlockSmem<SlKS, NA_T, Q>;
     auto fn = k_expand<S, SlKS, NA_T, Q>;
     fn<<<grid_of((const void*)fn, NA_T, L::bytes, (u64)(b - a) * NA_T, sms), NA_T, L::bytes, st>>>(in, start, a, b, offs, out,
-                                                                                      ticket, nullptr);
+                                                                                      ticket, nullptr, Ahead{});
 }
 
 template <int S>

@@ -51,7 +51,7 @@ template <class K> cudaError_t set_smem(K fn, int bytes)
 }
 
 template <int S, class SL, int T, bool SPARSE>
-cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem,
+cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem, const u32* n_dev,
                    cudaStream_t st, int sms)
 {
     constexpr int Q = QcapFor<SL, T>::leaf;
@@ -62,13 +62,13 @@ cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket,
     // a CTA for every node until the chip is full (node_chunk)
     static const int per_sm = resident_ctas((const void*)fn, T, L::bytes);
     const int grid = full_grid(per_sm, T, SPARSE ? n : (u64)n * T, sms);
-    fn<<<grid, T, L::bytes, st>>>(lv, start, n, acc, ticket, max_rem);
+    fn<<<grid, T, L::bytes, st>>>(lv, start, n, acc, ticket, max_rem, n_dev);
     return cudaGetLastError();
 }
 
 template <int S, class SL, int T>
 cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* offs, const LevelView& out, u32* ticket,
-                     cudaStream_t st, int sms)
+                     Ahead ahead, cudaStream_t st, int sms)
 {
     constexpr int Q = QcapFor<SL, T>::expand;
     using L = BlockSmem<SL, T, Q>;
@@ -77,34 +77,34 @@ cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* of
     if (attr) return attr;
     static const int per_sm = resident_ctas((const void*)fn, T, L::bytes);
     const int grid = full_grid(per_sm, T, (u64)(b - a) * T, sms);
-    fn<<<grid, T, L::bytes, st>>>(in, start, a, b, offs, out, ticket, nullptr);
+    fn<<<grid, T, L::bytes, st>>>(in, start, a, b, offs, out, ticket, nullptr, ahead);
     return cudaGetLastError();
 }
 
 template <class SL>
 cudaError_t leaf_any(int side, int T, const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem,
-                     bool sparse, cudaStream_t st, int sms)
+                     bool sparse, const u32* n_dev, cudaStream_t st, int sms)
 {
     if (sparse)
-        return side ? leaf_t<1, SL, 256, true>(lv, start, n, acc, ticket, max_rem, st, sms)
-                    : leaf_t<0, SL, 256, true>(lv, start, n, acc, ticket, max_rem, st, sms);
+        return side ? leaf_t<1, SL, 256, true>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms)
+                    : leaf_t<0, SL, 256, true>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms);
     if (T == 128)
-        return side ? leaf_t<1, SL, 128, false>(lv, start, n, acc, ticket, max_rem, st, sms)
-                    : leaf_t<0, SL, 128, false>(lv, start, n, acc, ticket, max_rem, st, sms);
+        return side ? leaf_t<1, SL, 128, false>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms)
+                    : leaf_t<0, SL, 128, false>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms);
     if (T == 512)
-        return side ? leaf_t<1, SL, 512, false>(lv, start, n, acc, ticket, max_rem, st, sms)
-                    : leaf_t<0, SL, 512, false>(lv, start, n, acc, ticket, max_rem, st, sms);
-    return side ? leaf_t<1, SL, 256, false>(lv, start, n, acc, ticket, max_rem, st, sms)
-                : leaf_t<0, SL, 256, false>(lv, start, n, acc, ticket, max_rem, st, sms);
+        return side ? leaf_t<1, SL, 512, false>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms)
+                    : leaf_t<0, SL, 512, false>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms);
+    return side ? leaf_t<1, SL, 256, false>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms)
+                : leaf_t<0, SL, 256, false>(lv, start, n, acc, ticket, max_rem, n_dev, st, sms);
 }
 
 template <class SL>
 cudaError_t expand_any(int side, int T, const LevelView& in, u32 start, u32 a, u32 b, const u64* offs,
-                       const LevelView& out, u32* ticket, cudaStream_t st, int sms)
+                       const LevelView& out, u32* ticket, Ahead ahead, cudaStream_t st, int sms)
 {
-    if (T == 128) return side ? expand_t<1, SL, 128>(in, start, a, b, offs, out, ticket, st, sms) : expand_t<0, SL, 128>(in, start, a, b, offs, out, ticket, st, sms);
-    if (T == 512) return side ? expand_t<1, SL, 512>(in, start, a, b, offs, out, ticket, st, sms) : expand_t<0, SL, 512>(in, start, a, b, offs, out, ticket, st, sms);
-    return side ? expand_t<1, SL, 256>(in, start, a, b, offs, out, ticket, st, sms) : expand_t<0, SL, 256>(in, start, a, b, offs, out, ticket, st, sms);
+    if (T == 128) return side ? expand_t<1, SL, 128>(in, start, a, b, offs, out, ticket, ahead, st, sms) : expand_t<0, SL, 128>(in, start, a, b, offs, out, ticket, ahead, st, sms);
+    if (T == 512) return side ? expand_t<1, SL, 512>(in, start, a, b, offs, out, ticket, ahead, st, sms) : expand_t<0, SL, 512>(in, start, a, b, offs, out, ticket, ahead, st, sms);
+    return side ? expand_t<1, SL, 256>(in, start, a, b, offs, out, ticket, ahead, st, sms) : expand_t<0, SL, 256>(in, start, a, b, offs, out, ticket, ahead, st, sms);
 }
 
 template <int S, class SL>
@@ -130,22 +130,22 @@ cudaError_t count_level_any(int side, const LevelView& lv, u32 start, u32 n, u32
 
 template <int S, class SL>
 cudaError_t count_plan_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap, PlanOut* plan,
-                         u32* done, const u32* err, cudaStream_t st)
+                         u32* done, const u32* err, Ahead ahead, cudaStream_t st)
 {
     auto fn = k_count_plan<S, SL>;
     constexpr int smem = table_smem_bytes<SL>();
     static cudaError_t attr = set_smem(fn, smem);
     if (attr) return attr;
-    fn<<<(n + 255) / 256, 256, smem, st>>>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err);
+    fn<<<(n + 255) / 256, 256, smem, st>>>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, ahead);
     return cudaGetLastError();
 }
 
 template <class SL>
 cudaError_t count_plan_any(int side, const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
-                           PlanOut* plan, u32* done, const u32* err, cudaStream_t st)
+                           PlanOut* plan, u32* done, const u32* err, Ahead ahead, cudaStream_t st)
 {
-    return side ? count_plan_t<1, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, st)
-                : count_plan_t<0, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, st);
+    return side ? count_plan_t<1, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, ahead, st)
+                : count_plan_t<0, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, ahead, st);
 }
 
 inline int small_grid(u32 n, int T) { return (int)std::max<u32>(1, std::min<u32>((n + T - 1) / T, 8192)); }

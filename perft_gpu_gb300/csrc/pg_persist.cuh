@@ -214,7 +214,7 @@ __device__ __forceinline__ void persist_plan(const u64* offs, u32 n, u64 cap, Pl
 template <int S>
 __device__ __forceinline__ void persist_leaf(const PersistArgs& A, int L, u32 start, u32 n, u32* ticket)
 {
-    leaf_body<S, SlKS, PERSIST_T, PERSIST_LEAF_Q, false>(A.lv[L], start, n, A.acc, ticket, 2u);
+    leaf_body<S, SlKS, PERSIST_T, PERSIST_LEAF_Q, false>(A.lv[L], start, n, A.acc, ticket, 2u, nullptr);
 }
 
 template <int S>

@@ -109,3 +109,28 @@ def test_small_calls_read_and_write_pinned_memory(pg, orc, n):
         boards, depths = pg.random_playouts(seed, n, 0, 60, 1, 0, 2, with_depths=True)
         want, _ = orc.perft_batch(boards, depths, os.cpu_count() or 1)
         assert np.array_equal(pg.perft_batch(boards, depths, persistent=persistent), want)
+
+
+# 224 legal moves: 294 of them have more children than the smallest level buffer
+BEYOND = "Q6Q/3Q4/1Q4Q1/4Q3/2Q4Q/Q4Q2/pp1Q4/kBNN1KB1 w - - 0 1"
+
+
+@pytest.mark.parametrize("n", [1, 2, 274, 300, 301])
+@pytest.mark.parametrize("depth", [3, 4])
+def test_levels_launched_before_their_size_is_known(pg, orc, n, depth):
+    """Up to 300 roots have their first levels launched without waiting for each
+    one's size; roots of every depth and both sides, and boards whose children do
+    not fit (the call then waits level by level)."""
+    want = {(f, d): orc.perft(orc.fen(f), d) for f in (MANY, BEYOND) for d in range(1, depth)}
+    assert want[BEYOND, 1] * 294 > 1 << 16
+    for fen in (MANY, BEYOND):
+        deep = min(depth, 3) if n > 1 else depth
+        boards, depths = _copies(pg, fen, n), np.full(n, deep, np.uint8)
+        expect = np.full(n, orc.perft(orc.fen(fen), deep), np.uint64)
+        if n > 250:
+            depths[::50] = 2
+            expect[::50] = want[fen, 2]
+        assert np.array_equal(pg.perft_batch(boards, depths), expect)
+    boards, depths = pg.random_playouts(61, n, 0, 60, 1, 0, depth, with_depths=True)
+    expect, _ = orc.perft_batch(boards, depths, os.cpu_count() or 1)
+    assert np.array_equal(pg.perft_batch(boards, depths), expect)
