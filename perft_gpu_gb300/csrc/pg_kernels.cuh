@@ -386,9 +386,13 @@ constexpr int LEAF_COLUMN = 48;  // queued moves a thread holds before they are 
 // children, ten (leaf) or thirty (expansion) a node, on all of them, where a full
 // chunk would leave SMs idle and give every thread its nodes' children one after
 // the other.
-__device__ __forceinline__ u32 node_chunk(u32 n, u32 threads)
+struct Share {
+    u32 cta, ctas;  // which of the CTAs that work on these nodes this one is
+};
+__device__ __forceinline__ Share whole_grid() { return Share{blockIdx.x, gridDim.x}; }
+__device__ __forceinline__ u32 node_chunk(u32 n, u32 threads, const Share& sh)
 {
-    const u32 even = (n + gridDim.x - 1) / gridDim.x;
+    const u32 even = (n + sh.ctas - 1) / sh.ctas;
     return min(threads, even <= 32u ? even : (even + 31u) & ~31u);
 }
 
@@ -424,7 +428,7 @@ template <int T> constexpr int min_blocks() { return (PG_LEAF_MIN_WARPS * 32 + T
 // same grp[] / rem[] subscripts and a load_board overload.
 template <int S, class SL, int T, int QCAP, bool SPARSE, class LV>
 __device__ __forceinline__ void leaf_body(LV lv, u32 start, u32 n, u64* __restrict__ acc, u32* ticket, u32 max_rem,
-                                          const u32* n_dev)
+                                          const u32* n_dev, const Share share)
 {
     extern __shared__ __align__(16) unsigned char pg_dyn_smem[];
 #include "pg_leaf_body.inc"
@@ -436,6 +440,7 @@ __global__ void __launch_bounds__(T, min_blocks<T>()) k_leaf(LevelView lv, u32 s
 {
     extern __shared__ __align__(16) unsigned char pg_dyn_smem[];
     stage_tables<SL>();
+    const Share share = whole_grid();
 #include "pg_leaf_body.inc"
 }
 
@@ -445,7 +450,7 @@ __global__ void __launch_bounds__(T, min_blocks<T>()) k_leaf(LevelView lv, u32 s
 // slot and its parent's slot is written to parent_out
 template <int S, class SL, int T, int QCAP>
 __device__ __forceinline__ void expand_body(const LevelView& in, u32 start, u32 a, u32 b, const u64* offs,
-                                            const LevelView& out, u32* ticket, u32* parent_out)
+                                            const LevelView& out, u32* ticket, u32* parent_out, const Share share)
 {
     extern __shared__ __align__(16) unsigned char pg_dyn_smem[];
     using L = BlockSmem<SL, T, QCAP>;
@@ -456,7 +461,7 @@ __device__ __forceinline__ void expand_body(const LevelView& in, u32 start, u32 
     __shared__ u32 s_chunk;
     const int tid = threadIdx.x;
     const u64 out_base = offs[a];
-    const u32 per = node_chunk(b - a, T);
+    const u32 per = node_chunk(b - a, T, share);
     for (;;) {
         if (tid == 0) s_chunk = atomicAdd(ticket, 1u);
         __syncthreads();
@@ -520,7 +525,7 @@ __global__ void __launch_bounds__(T, min_blocks<T>()) k_expand(LevelView in, u32
         if (*ahead.children == 0) return;  // none, or more than `out` holds
         if (ahead.nodes) b = *ahead.nodes;
     }
-    expand_body<S, SL, T, QCAP>(in, start, a, b, offs, out, ticket, parent_out);
+    expand_body<S, SL, T, QCAP>(in, start, a, b, offs, out, ticket, parent_out, whole_grid());
 }
 
 }  // namespace pg

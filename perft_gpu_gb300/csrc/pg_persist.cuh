@@ -214,13 +214,13 @@ __device__ __forceinline__ void persist_plan(const u64* offs, u32 n, u64 cap, Pl
 template <int S>
 __device__ __forceinline__ void persist_leaf(const PersistArgs& A, int L, u32 start, u32 n, u32* ticket)
 {
-    leaf_body<S, SlKS, PERSIST_T, PERSIST_LEAF_Q, false>(A.lv[L], start, n, A.acc, ticket, 2u, nullptr);
+    leaf_body<S, SlKS, PERSIST_T, PERSIST_LEAF_Q, false>(A.lv[L], start, n, A.acc, ticket, 2u, nullptr, whole_grid());
 }
 
 template <int S>
 __device__ __forceinline__ void persist_expand(const PersistArgs& A, int L, u32 start, u32 a, u32 b, u32* ticket)
 {
-    expand_body<S, SlKS, PERSIST_T, PERSIST_Q>(A.lv[L], start, a, b, A.offs[L], A.lv[L + 1], ticket, nullptr);
+    expand_body<S, SlKS, PERSIST_T, PERSIST_Q>(A.lv[L], start, a, b, A.offs[L], A.lv[L + 1], ticket, nullptr, whole_grid());
 }
 
 template <int S>

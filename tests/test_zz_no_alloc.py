@@ -86,3 +86,24 @@ def test_noalloc_rejects_sizes_beyond_its_maximum():
     st, out, _, _ = _call(fn, boards, np.full(len(boards), 3, np.uint8))
     assert st == PG_ERR_CAPACITY
     assert not out.any()
+
+
+@pytest.mark.parametrize("white, black", [(1, 0), (0, 1), (1, 1), (303, 1), (2, 303), (152, 152), (5000, 1), (0, 700), (9000, 11000)])
+def test_noalloc_sides_share_launches(white, black):
+    """Both sides' nodes go through one launch a level: one side empty, one
+    node against many, sizes about a round of the SMs."""
+    pg, fn = _entry()
+    pg.init()
+    b, d = pg.random_playouts(67, 4 * (white + black) + 64, 0, 60, 1, 0, 3, with_depths=True)
+    is_black = (b["pawns"] >> np.uint64(63)) != 0
+    keep = np.sort(np.concatenate([np.flatnonzero(~is_black)[:white], np.flatnonzero(is_black)[:black]]))
+    b, d = b[keep].copy(), d[keep].copy()
+    assert len(b) == white + black
+    want = pg.perft_batch(b, d, slider="ks")
+    for depths in (d, np.minimum(d, 2)):
+        st, got, _, _ = _call(fn, b, depths)
+        assert st == 0
+        if depths is d:
+            assert np.array_equal(got, want)
+        else:
+            assert np.array_equal(got, pg.perft_batch(b, depths, slider="ks"))
