@@ -1273,7 +1273,7 @@ static int init_locked(Engine& E, const pg_config* cfg)
     PG_CUDA(cudaMalloc(&E.plan_dev, sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.plan_host, (1 + AHEAD_PLANS) * sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.host_scratch, 4096));
-    PG_CUDA(cudaMallocHost(&E.host_io, HOST_IO_ROOTS * (48 + 1 + 8) + 64));
+    PG_CUDA(cudaMallocHost(&E.host_io, HOST_IO_BYTES));
     PG_CUDA(cudaMalloc(&E.aux, 256));
     PG_CUDA(cudaDeviceSynchronize());
     E.ready = true;
@@ -1305,17 +1305,27 @@ static int op_batch(int op, const pg_board* pos, u32 n, void* out, u32* nout, in
     const u64 in_bytes = (u64)n * sizeof(Pos);
     const u64 out_bytes = op == 0 ? (u64)n * 4 : op == 1 ? (u64)n * 512 : (u64)n * 256 * sizeof(Pos);
     const u64 nbytes = (u64)n * 4;
-    PG_TRY(ensure_stage(in_bytes + out_bytes + nbytes + 64));
-    unsigned char* s = (unsigned char*)E.stage;
+    // a small call's kernel reads and writes pinned memory: no copies of its own
+    // (one position's moves 37 -> 18 us, its number of moves 18 -> 13 us)
+    const bool in_place = in_bytes + out_bytes + nbytes <= HOST_IO_BYTES;
+    if (!in_place) PG_TRY(ensure_stage(in_bytes + out_bytes + nbytes + 64));
+    unsigned char* s = in_place ? E.host_io : (unsigned char*)E.stage;
     Pos* d_in = (Pos*)s;
     void* d_out = s + in_bytes;
     u32* d_n = (u32*)(s + in_bytes + out_bytes);
-    PG_CUDA(cudaMemcpyAsync(d_in, pos, in_bytes, cudaMemcpyHostToDevice, E.stream));
+    if (in_place) memcpy(d_in, pos, in_bytes);
+    else PG_CUDA(cudaMemcpyAsync(d_in, pos, in_bytes, cudaMemcpyHostToDevice, E.stream));
     if (check) PG_TRY(check_roots_device(d_in, nullptr, pos, nullptr, n));
     const SliderOps& ops = ops_for(slider);
     if (op == 0) PG_CUDA(ops.count_batch(d_in, n, (u32*)d_out, E.stream));
     else if (op == 1) PG_CUDA(ops.gen_moves_batch(d_in, n, (u16*)d_out, d_n, E.stream));
     else PG_CUDA(ops.gen_boards_batch(d_in, n, (Pos*)d_out, d_n, E.stream));
+    if (in_place) {
+        PG_CUDA(cudaStreamSynchronize(E.stream));
+        memcpy(out, d_out, out_bytes);
+        if (nout) memcpy(nout, d_n, nbytes);
+        return PG_OK;
+    }
     PG_CUDA(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, E.stream));
     if (nout) PG_CUDA(cudaMemcpyAsync(nout, d_n, nbytes, cudaMemcpyDeviceToHost, E.stream));
     PG_CUDA(cudaStreamSynchronize(E.stream));
@@ -1624,15 +1634,13 @@ int pg_perft_divide(const pg_board* pos, int depth, pg_move* moves, uint64_t* co
     {
         Engine& E = engine();
         std::lock_guard<std::mutex> lk(E.mu);
-        PG_TRY(ensure_stage(256 * 48 + 512 + 64));
-        Pos* d = (Pos*)E.stage;
-        u16* dm = (u16*)((unsigned char*)E.stage + 256 * 48);
-        for (u32 i = 0; i < *n; i++) kids[i] = *pos;
-        PG_CUDA(cudaMemcpyAsync(d, kids, *n * 48, cudaMemcpyHostToDevice, E.stream));
-        PG_CUDA(cudaMemcpyAsync(dm, moves, *n * 2, cudaMemcpyHostToDevice, E.stream));
+        Pos* d = (Pos*)E.host_io;
+        u16* dm = (u16*)(E.host_io + 256 * 48);
+        for (u32 i = 0; i < *n; i++) memcpy(d + i, pos, sizeof(Pos));
+        memcpy(dm, moves, *n * 2);
         PG_CUDA(g_ops_ks.make_batch(d, dm, *n, E.stream));
-        PG_CUDA(cudaMemcpyAsync(kids, d, *n * 48, cudaMemcpyDeviceToHost, E.stream));
         PG_CUDA(cudaStreamSynchronize(E.stream));
+        memcpy(kids, d, *n * 48);
     }
     uint8_t dep[256];
     for (u32 i = 0; i < *n; i++) dep[i] = (uint8_t)(depth - 1);

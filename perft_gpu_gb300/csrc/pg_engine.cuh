@@ -24,6 +24,7 @@ constexpr u32 AHEAD_MOVES = 218;
 constexpr u32 AHEAD_NODES = 1u << 16;
 constexpr int AHEAD_PLANS = 4;  // two levels for each side of the roots (1 x 218 x 218 is under AHEAD_NODES)
 constexpr u32 HOST_IO_ROOTS = 4096;   // largest host-array call staged in pinned memory and checked on the host
+constexpr u32 HOST_IO_BYTES = HOST_IO_ROOTS * (48 + 1 + 8) + 64;
 constexpr u32 MAX_TICKETS = 1 << 16;  // dynamic-scheduling counters per call
 
 // device error bits (bounded waits and capacity guards set them; no trap)

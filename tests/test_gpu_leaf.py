@@ -134,3 +134,17 @@ def test_levels_launched_before_their_size_is_known(pg, orc, n, depth):
     boards, depths = pg.random_playouts(61, n, 0, 60, 1, 0, depth, with_depths=True)
     expect, _ = orc.perft_batch(boards, depths, os.cpu_count() or 1)
     assert np.array_equal(pg.perft_batch(boards, depths), expect)
+
+
+@pytest.mark.parametrize("n", [1, 4096, 4097, 4170, 4171])
+def test_operator_calls_at_the_pinned_buffer_s_size(pg, orc, n):
+    """Boards and results of up to 4,170 positions fit the pinned buffer."""
+    boards = pg.random_playouts(71, n, 0, 60)
+    want, _ = orc.perft_batch(boards, np.full(n, 1, np.uint8), os.cpu_count() or 1)
+    assert np.array_equal(pg.count_moves_batch(boards).astype(np.uint64), want)
+    pos = pg.board_of(boards[n // 2])
+    assert len(pg.generate_moves(pos)) == len(pg.generate_boards(pos)) == want[n // 2]
+    divided = pg.perft_divide(pos, 2)
+    assert [m for m, _ in divided] == list(pg.generate_moves(pos))
+    total, _ = orc.perft_batch(boards[n // 2:n // 2 + 1], np.full(1, 2, np.uint8), 1)
+    assert sum(c for _, c in divided) == total[0]
