@@ -48,13 +48,11 @@ struct TTSet {
 };
 
 struct LevelTT {
-    u64* hash0 = nullptr;  // 128-bit key of each node, low / high word
-    u64* hash1 = nullptr;
+    ulonglong2* key = nullptr;  // 128-bit key of each node
     u64* acc = nullptr;
     u32* parent = nullptr;
     u32* dup = nullptr;
-    u64* dd_hash = nullptr;  // duplicate table of the level
-    u32* dd_idx = nullptr;
+    u64* dd = nullptr;  // duplicate table of the level: claims (dd_claim), ~0 where empty
     u64 cap = 0, dd_cap = 0;
     void* block = nullptr;
 };
@@ -85,6 +83,18 @@ __device__ __forceinline__ u64 dd_key(u64 h, u32 rem)
     const u64 k = h ^ (0x9E3779B97F4A7C15ull * (rem + 1));
     return k ? k : 1;
 }
+// What a node writes to its slot, the least winning: 32 bits of the digest over
+// the node's index.  The claimant of a slot is the lowest index among the nodes
+// of the least digest.  One word and one reduction a node, 3 slots a node: as a
+// digest claimed by compare-and-swap and an index beside it (two sectors a node,
+// 2 slots in the same bytes) the probe of 64 positions at depth 6 took 2.92 ms and
+// the comparison 1.47 ms, so 1.92 and 1.04, and the leaf 0.4 ms less for the
+// duplicates that no longer lose their slot to another position; both kernels
+// wait for random sectors, and with the two key words of a node side by side, the
+// depths compared only where a level mixes them, and the key update square by
+// square (zobrist128_from) they take 1.72 and 0.88 ms.
+__device__ __forceinline__ u64 dd_claim(u64 k, u32 idx) { return k << 32 | idx; }
+constexpr int DD_SLOTS = 3;  // slots a node
 // slot of a digest in a table of `slots` entries (any size): the high word of
 // digest x slots, after a multiply that spreads every digest bit upward
 __device__ __forceinline__ u32 dd_slot(u64 k, u64 slots)
@@ -110,8 +120,7 @@ __device__ __forceinline__ void block_count_add(u64* dst, u32 v)
 // boards and keys, and each node's parent slot (parent null at the root level)
 struct ParentKeys {
     LevelView lv;
-    const u64* hash0;
-    const u64* hash1;
+    const ulonglong2* key;
     const u32* parent;
 };
 
@@ -138,12 +147,11 @@ static __global__ void k_tt_probe(LevelView lv, u32 start, u32 n, LevelTT lt, Pa
         if (pk.parent) {
             const u32 p = pk.parent[idx];
             const Pos pb = load_board(pk.lv, p);
-            h = zobrist128_from(&pb.w, make_ulonglong2(pk.hash0[p], pk.hash1[p]), &b.w, z);
+            h = zobrist128_from(&pb.w, pk.key[p], &b.w, z);
         } else {
             h = zobrist128(&b.w, z);
         }
-        lt.hash0[idx] = h.x;
-        lt.hash1[idx] = h.y;
+        lt.key[idx] = h;
         if (rem <= TT_MAX_DEPTH && tt.tab[rem]) {
             probes++;
             const ulonglong2* e = tt.tab[rem] + 2 * (h.x & tt.mask[rem]);
@@ -158,8 +166,7 @@ static __global__ void k_tt_probe(LevelView lv, u32 start, u32 n, LevelTT lt, Pa
         }
         const u64 k = dd_key(h.x, rem);
         const u32 s = dd_slot(k, dd_slots);
-        const u64 prev = atomicCAS(&lt.dd_hash[s], 0ull, k);
-        if (prev == 0 || prev == k) atomicMin(&lt.dd_idx[s], idx);
+        atomicMin(&lt.dd[s], dd_claim(k, idx));
     }
     block_count_add(&counters[0], probes);
     block_count_add(&counters[1], hits);
@@ -171,20 +178,25 @@ static __global__ void k_tt_probe(LevelView lv, u32 start, u32 n, LevelTT lt, Pa
 // slot's digest; a node whose full key or depth differs from the claimant's
 // (a digest collision) keeps its own work.  Claimants are never marked here,
 // so their depth and key are stable while others compare against them.
-static __global__ void k_tt_dedup(LevelView lv, u32 start, u32 n, LevelTT lt, u64 dd_slots)
+// one_rem: every live node of the level has the same remaining depth.
+static __global__ void k_tt_dedup(LevelView lv, u32 start, u32 n, LevelTT lt, u64 dd_slots, bool one_rem)
 {
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const u32 idx = start + i;
         const u32 rem = lv.rem[idx];
         if (rem < TT_MIN_DEPTH || rem >= REM_DEAD) continue;
-        const u64 h0 = lt.hash0[idx];
-        const u64 k = dd_key(h0, rem);
+        const ulonglong2 h = lt.key[idx];
+        const u64 k = dd_key(h.x, rem);
         const u32 s = dd_slot(k, dd_slots);
-        if (lt.dd_hash[s] == k) {
-            const u32 rep = lt.dd_idx[s];
-            if (rep != idx && lt.hash0[rep] == h0 && lt.hash1[rep] == lt.hash1[idx] && lv.rem[rep] == rem) {
-                lt.dup[idx] = rep;
-                lv.rem[idx] = REM_DEAD;
+        const u64 claim = lt.dd[s];
+        if ((u32)(claim >> 32) == (u32)k) {
+            const u32 rep = (u32)claim;
+            if (rep != idx) {
+                const ulonglong2 r = lt.key[rep];
+                if (r.x == h.x && r.y == h.y && (one_rem || lv.rem[rep] == rem)) {
+                    lt.dup[idx] = rep;
+                    lv.rem[idx] = REM_DEAD;
+                }
             }
         }
     }
@@ -221,7 +233,8 @@ static __global__ void k_tt_upsweep(LevelView ch, u32 m, LevelTT ct, TTSet tt, u
             v = d != NO_DUP ? ct.acc[d] : ct.acc[j];
             const u32 rem = ch.rem[j];
             if (rem >= TT_MIN_DEPTH && rem <= TT_MAX_DEPTH && tt.tab[rem]) {
-                tt_store(tt, rem, ct.hash0[j], ct.hash1[j], v);
+                const ulonglong2 h = ct.key[j];
+                tt_store(tt, rem, h.x, h.y, v);
                 stores++;
             }
             par = ct.parent[j];
@@ -260,7 +273,7 @@ static __global__ void k_tt_finish(LevelView lv, u32 n, LevelTT lt, TTSet tt, co
         const u64 v = d != NO_DUP ? lt.acc[d] : lt.acc[s];
         const u32 rem = lv.rem[s];
         if (rem >= TT_MIN_DEPTH && rem <= TT_MAX_DEPTH && tt.tab[rem]) {
-            tt_store(tt, rem, lt.hash0[s], lt.hash1[s], v);
+            tt_store(tt, rem, lt.key[s].x, lt.key[s].y, v);
             stores++;
         }
         out[root_of[s]] = v;
@@ -331,9 +344,9 @@ static int ensure_tables(u64 bytes)
 }
 
 // per node of a level in the TT driver, beside the level buffer: both key
-// words, the count, the parent slot and the duplicate index (32 B), and two
-// slots of the level's duplicate table (12 B each)
-constexpr u64 TT_NODE_BYTES = 32 + 2 * 12;
+// words, the count, the parent slot and the duplicate index (32 B), and its
+// slots of the level's duplicate table (8 B each)
+constexpr u64 TT_NODE_BYTES = 32 + DD_SLOTS * 8;
 
 // nodes a level of the TT driver holds: a quarter of the HBM budget left
 // beside the tables, over the level buffer's and the TT metadata's bytes
@@ -358,8 +371,8 @@ static int ensure_level_tt(int L, u64 need)
         t = LevelTT{};
     }
     const u64 cap = std::max<u64>(1u << 16, (need + 65535) & ~65535ull);
-    const u64 dd = 2 * cap;
-    const u64 bytes = cap * (8 + 8 + 8 + 4 + 4) + dd * (8 + 4) + 1024;
+    const u64 dd = DD_SLOTS * cap;
+    const u64 bytes = cap * (8 + 8 + 8 + 4 + 4) + dd * 8 + 1024;
     void* blk = nullptr;
     cudaError_t e = cudaMalloc(&blk, bytes);
     if (e != cudaSuccess) {
@@ -369,19 +382,16 @@ static int ensure_level_tt(int L, u64 need)
         return PG_ERR_OUT_OF_MEMORY;
     }
     unsigned char* p = (unsigned char*)blk;
-    t.hash0 = (u64*)p;
-    p += cap * 8;
-    t.hash1 = (u64*)p;
-    p += cap * 8;
+    t.key = (ulonglong2*)p;
+    p += cap * 16;
     t.acc = (u64*)p;
     p += cap * 8;
-    t.dd_hash = (u64*)p;
+    t.dd = (u64*)p;
     p += dd * 8;
     t.parent = (u32*)p;
     p += cap * 4;
     t.dup = (u32*)p;
     p += cap * 4;
-    t.dd_idx = (u32*)p;
     t.cap = cap;
     t.dd_cap = dd;
     t.block = blk;
@@ -394,15 +404,14 @@ static int run_range_tt(const Variant& v, int L, u32 start, u32 n, int side, int
     if (n == 0) return PG_OK;
     LevelBuf& lb = E.lv[L];
     LevelTT& lt = g_tt.lv[L];
-    // two duplicate-table slots per node of the range (the table is sized for
+    // duplicate-table slots for the nodes of the range (the table is sized for
     // the level's capacity)
-    const u64 dd = std::min(std::max<u64>(1024, 2ull * n), lt.dd_cap);
-    TT_CUDA(cudaMemsetAsync(lt.dd_hash, 0, dd * 8, E.stream));
-    TT_CUDA(cudaMemsetAsync(lt.dd_idx, 0xFF, dd * 4, E.stream));
+    const u64 dd = std::min(std::max<u64>(1024, (u64)DD_SLOTS * n), lt.dd_cap);
+    TT_CUDA(cudaMemsetAsync(lt.dd, 0xFF, dd * 8, E.stream));
     ParentKeys pk{};
-    if (L > 0) pk = {E.lv[L - 1].v, g_tt.lv[L - 1].hash0, g_tt.lv[L - 1].hash1, lt.parent};
+    if (L > 0) pk = {E.lv[L - 1].v, g_tt.lv[L - 1].key, lt.parent};
     k_tt_probe<<<small_grid(n), 256, 0, E.stream>>>(lb.v, start, n, lt, pk, g_tt.active, dd, g_tt.counters);
-    k_tt_dedup<<<small_grid(n), 256, 0, E.stream>>>(lb.v, start, n, lt, dd);
+    k_tt_dedup<<<small_grid(n), 256, 0, E.stream>>>(lb.v, start, n, lt, dd, minrem == maxrem);
     TT_CUDA(cudaGetLastError());
     E.st.launches += 2;
     if (minrem <= 2) TT_TRY(launch_leaf(v, side, lb.v, start, n, lt.acc, true));

@@ -119,21 +119,23 @@ __host__ __device__ __forceinline__ ulonglong2 zobrist128_from(const u64* pw, ul
 {
     if (kp.x == 1 && kp.y == 0) return zobrist128(cw, z);
     const u64 pp = pw[1] & 0x00FFFFFFFFFFFF00ull, cp = cw[1] & 0x00FFFFFFFFFFFF00ull;
-    const u64 ps[6] = {pp, pw[2], pw[3] & ~pw[4], pw[4] & ~pw[3], pw[3] & pw[4], pw[5]};
-    const u64 cs[6] = {cp, cw[2], cw[3] & ~cw[4], cw[4] & ~cw[3], cw[3] & cw[4], cw[5]};
     u64 h0 = kp.x, h1 = kp.y;
-#pragma unroll
-    for (int t = 0; t < 6; t++) {
-        for (u64 s = (ps[t] & pw[0]) ^ (cs[t] & cw[0]); s; s &= s - 1) {
-            const ulonglong2 e = z[t * 64 + zb_lsb(s)];
-            h0 ^= e.x;
-            h1 ^= e.y;
-        }
-        for (u64 s = (ps[t] & ~pw[0]) ^ (cs[t] & ~cw[0]); s; s &= s - 1) {
-            const ulonglong2 e = z[(6 + t) * 64 + zb_lsb(s)];
-            h0 ^= e.x;
-            h1 ^= e.y;
-        }
+    // square by square, what left it and what came: two squares for most moves,
+    // so the lanes of a warp stay together (with a loop a piece set nearly each of
+    // the twelve has a feature of some lane)
+    auto piece = [&](u64 bit, const u64* b, u64 pawns, int s) {
+        if (!((pawns | b[2] | b[3] | b[4] | b[5]) & bit)) return;
+        const int bq = (b[3] & bit) != 0, rq = (b[4] & bit) != 0;
+        const int t = ((b[2] & bit) != 0) + 2 * bq + 3 * rq - (bq & rq) + ((b[5] & bit) ? 5 : 0) + ((b[0] & bit) ? 0 : 6);
+        const ulonglong2 e = z[t * 64 + s];
+        h0 ^= e.x;
+        h1 ^= e.y;
+    };
+    for (u64 d = (pw[0] ^ cw[0]) | (pp ^ cp) | (pw[2] ^ cw[2]) | (pw[3] ^ cw[3]) | (pw[4] ^ cw[4]) | (pw[5] ^ cw[5]); d; d &= d - 1) {
+        const u64 bit = d & (0 - d);
+        const int s = zb_lsb(d);
+        piece(bit, pw, pp, s);
+        piece(bit, cw, cp, s);
     }
     const u64 ds = pw[1] ^ cw[1];
 #pragma unroll

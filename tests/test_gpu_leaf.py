@@ -148,3 +148,17 @@ def test_operator_calls_at_the_pinned_buffer_s_size(pg, orc, n):
     assert [m for m, _ in divided] == list(pg.generate_moves(pos))
     total, _ = orc.perft_batch(boards[n // 2:n // 2 + 1], np.full(1, 2, np.uint8), 1)
     assert sum(c for _, c in divided) == total[0]
+
+
+@pytest.mark.parametrize("lo, hi", [(4, 4), (3, 5)])
+def test_duplicates_within_and_across_depths(pg, orc, lo, hi):
+    """The duplicate pass takes a node's depth into account where a level mixes
+    depths: the same positions at several depths, and once more each."""
+    boards = pg.random_playouts(73, 40, 4, 40)
+    boards = np.concatenate([boards] * (2 * (hi - lo + 1)))
+    depths = np.repeat(np.arange(lo, hi + 1, dtype=np.uint8), 80)
+    want, _ = orc.perft_batch(boards, depths, os.cpu_count() or 1)
+    for mode in ("dedup", True):
+        pg.tt_clear()
+        assert np.array_equal(pg.perft_batch(boards, depths, use_tt=mode, tt_bytes=1 << 28), want)
+    pg.tt_clear()
