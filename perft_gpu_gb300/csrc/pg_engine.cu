@@ -319,14 +319,11 @@ static int run_children(const Variant& v, int L, u32 start, u32 n, int side, int
             if (n_dev) n = plan.bnd[1];
         }
         if (!fused || (plan.nchunks == 0 && !errv)) {
-            k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_dev, E.err);
+            k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_host, E.err);
             PG_CUDA(cudaGetLastError());
             E.st.launches++;
-            u32* perr = (u32*)(E.host_scratch + 192);  // pinned
-            PG_CUDA(cudaMemcpyAsync(E.plan_host, E.plan_dev, sizeof(PlanOut), cudaMemcpyDeviceToHost, E.stream));
-            PG_CUDA(cudaMemcpyAsync(perr, E.err, sizeof(u32), cudaMemcpyDeviceToHost, E.stream));
             PG_CUDA(cudaStreamSynchronize(E.stream));
-            errv = *perr;
+            errv = plan.pad;
         }
         collect_leaf_timers();
         if (errv) {
@@ -1199,7 +1196,6 @@ static void release_engine(Engine& E)
     if (E.scan_status) cudaFree(E.scan_status);
     if (E.stage) cudaFree(E.stage);
     if (E.tickets) cudaFree(E.tickets);
-    if (E.plan_dev) cudaFree(E.plan_dev);
     if (E.plan_host) cudaFreeHost(E.plan_host);
     if (E.host_scratch) cudaFreeHost(E.host_scratch);
     if (E.host_io) cudaFreeHost(E.host_io);
@@ -1221,7 +1217,6 @@ static void release_engine(Engine& E)
     E.tickets = nullptr;
     E.err = nullptr;
     E.ahead_n = nullptr;
-    E.plan_dev = nullptr;
     E.plan_host = nullptr;
     E.host_scratch = nullptr;
     E.aux = nullptr;
@@ -1270,7 +1265,6 @@ static int init_locked(Engine& E, const pg_config* cfg)
     PG_CUDA(cudaMalloc(&E.tickets, (MAX_TICKETS + 4 + AHEAD_PLANS) * sizeof(u32)));
     E.err = E.tickets + MAX_TICKETS;
     E.ahead_n = E.err + 4;
-    PG_CUDA(cudaMalloc(&E.plan_dev, sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.plan_host, (1 + AHEAD_PLANS) * sizeof(PlanOut)));
     PG_CUDA(cudaMallocHost(&E.host_scratch, 4096));
     PG_CUDA(cudaMallocHost(&E.host_io, HOST_IO_BYTES));

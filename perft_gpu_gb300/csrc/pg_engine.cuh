@@ -151,7 +151,6 @@ struct Engine {
     u32* tickets = nullptr;  // MAX_TICKETS counters, zeroed per call
     u32 ticket_next = 0;
     u32* err = nullptr;      // error bits, the word behind the counters (cleared with them)
-    PlanOut* plan_dev = nullptr;
     PlanOut* plan_host = nullptr;  // pinned: the plan waited for, then one for each level launched ahead
     u32* ahead_n = nullptr;        // nodes of the levels launched ahead
     int ahead_plans = 0;           // how many the call has launched

@@ -193,15 +193,25 @@ static __global__ void __launch_bounds__(SCAN_T) k_scan(const u32* __restrict__ 
     if ((u64)tile * SCAN_TILE + SCAN_TILE >= n && tid == SCAN_T - 1) out[n] = s_prefix + aggregate;
 }
 
-// greedy chunking: consecutive node ranges whose children fit `cap`
+// greedy chunking: consecutive node ranges whose children fit `cap`.  The plan
+// goes to pinned host memory, pad: the error bits; most levels fit whole, which
+// the last offset tells without a search (17 dependent reads over 100,000 nodes:
+// the kernel 9.3 -> 3.3 us, and no copies behind it).
 static __global__ void k_plan(const u64* __restrict__ offs, u32 n, u64 cap, PlanOut* plan, u32* err)
 {
     if (threadIdx.x || blockIdx.x) return;
     u32 a = 0, k = 0;
+    const u64 total = offs[n];
     plan->bnd[0] = 0;
     plan->coff[0] = offs[0];
     while (a < n && k < MAX_CHUNKS) {
         const u64 limit = offs[a] + cap;
+        if (total <= limit) {
+            plan->bnd[++k] = n;
+            plan->coff[k] = total;
+            a = n;
+            break;
+        }
         u32 lo = a + 1, hi = n;  // largest b in [a+1, n] with offs[b] <= limit
         if (offs[lo] > limit) {
             hi = lo;  // one node alone exceeds the cap; cannot happen for cap >= 256
@@ -217,7 +227,8 @@ static __global__ void k_plan(const u64* __restrict__ offs, u32 n, u64 cap, Plan
     }
     if (a < n) atomicOr(err, ERR_PLAN_OVERFLOW);
     plan->nchunks = k;
-    plan->total = offs[n];
+    plan->pad = atomicOr(err, 0u);
+    plan->total = total;
 }
 
 // largest depth of a batch (out zeroed by the caller)

@@ -187,10 +187,17 @@ __device__ __forceinline__ void persist_scan(const u32* in, u32 n, u64* out, u64
 __device__ __forceinline__ void persist_plan(const u64* offs, u32 n, u64 cap, PlanOut* plan, u32* err)
 {
     u32 a = 0, k = 0;
+    const u64 total = offs[n];
     plan->bnd[0] = 0;
     plan->coff[0] = offs[0];
     while (a < n && k < MAX_CHUNKS) {
         const u64 limit = offs[a] + cap;
+        if (total <= limit) {
+            plan->bnd[++k] = n;
+            plan->coff[k] = total;
+            a = n;
+            break;
+        }
         u32 lo = a + 1, hi = n;  // largest b in [a+1, n] with offs[b] <= limit
         if (offs[lo] > limit) {
             hi = lo;  // one node alone exceeds the cap (caps are >= 65,536 > 256 moves)
@@ -206,7 +213,7 @@ __device__ __forceinline__ void persist_plan(const u64* offs, u32 n, u64 cap, Pl
     }
     if (a < n) atomicOr(err, ERR_PLAN_OVERFLOW);
     plan->nchunks = k;
-    plan->total = offs[n];
+    plan->total = total;
 }
 
 // the phases are inlined into the kernel: as called functions the leaf phase

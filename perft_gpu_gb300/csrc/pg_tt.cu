@@ -419,11 +419,10 @@ static int run_range_tt(const Variant& v, int L, u32 start, u32 n, int side, int
     TT_TRY(launch_count(v, side, lb.v, start, n, lb.cnt));
     TT_TRY(launch_scan(lb.cnt, n, lb.offs));
     const u64 cap_next = tt_level_cap();
-    k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_dev, E.err);
+    k_plan<<<1, 32, 0, E.stream>>>(lb.offs, n, cap_next, E.plan_host, E.err);
     TT_CUDA(cudaGetLastError());
-    TT_CUDA(cudaMemcpyAsync(E.plan_host, E.plan_dev, sizeof(PlanOut), cudaMemcpyDeviceToHost, E.stream));
     TT_CUDA(cudaStreamSynchronize(E.stream));
-    const PlanOut plan = *E.plan_host;
+    const PlanOut& plan = *E.plan_host;  // copied out here: deeper levels reuse the pinned buffer
     std::vector<u32> bnd(plan.bnd, plan.bnd + plan.nchunks + 1);
     std::vector<u64> boff(plan.coff, plan.coff + plan.nchunks + 1);
     const int cminrem = std::max(minrem, 3) - 1, cmaxrem = maxrem - 1;
