@@ -22,7 +22,7 @@ else the oracle's C restatement of it, on the same fixed sample of the
 workload every step (every 16th position, the sample of the cpu_baseline leg).
 
 --profile-case N runs every (4096/N)-th position of the workload once
-(Kogge-Stone sliders, 128-thread CTAs, two-ply leaf: the autotuner's choice
+(Kogge-Stone sliders, 256-thread CTAs, two-ply leaf: the autotuner's choice
 for the depths that hold most leaves; with --persistent as one persistent
 launch), checks the counts and prints one JSON line: the small case of the
 same kernels for ncu captures.
@@ -589,7 +589,7 @@ def run_ours(args):
         assert int(d_out.cpu().numpy().view(np.uint64).sum()) == leaves_per_step
         persist[name] = {"value": leaves_per_step * psteps * world / el, "unit": "leaf nodes/s",
                          "ms_per_step": 1e3 * el / psteps, "steps": psteps}
-    persist["note"] = ("one cooperative persistent launch per step (Kogge-Stone, 128-thread CTAs, two-ply leaf); "
+    persist["note"] = ("one cooperative persistent launch per step (Kogge-Stone, 256-thread CTAs, two-ply leaf); "
                        "'graph': that launch replayed from a captured graph (valid for any contents)")
 
     # the same steps with the in-level duplicate pass (use_tt="dedup": no
@@ -761,7 +761,7 @@ def run_profile_case(args):
     if args.persistent:
         out = pg.perft_batch(boards[idx], depths[idx], persistent=True, stats=st)
     else:
-        out = pg.perft_batch(boards[idx], depths[idx], slider="ks", block_size=128, leaf_plies=2, stats=st)
+        out = pg.perft_batch(boards[idx], depths[idx], slider="ks", block_size=256, leaf_plies=2, stats=st)
     ok = bool(np.array_equal(out, g[0][idx])) if g is not None else None
     print(json.dumps({"profile_case": len(idx), "persistent": bool(args.persistent),
                       "positions": "every %dth of the batched workload" % (len(boards) // len(idx)),

@@ -260,7 +260,7 @@ typedef struct pg_server_config {
     uint32_t max_inflight;       /* request slots; 0 = 4096 */
     int slider;
     uint32_t max_wave_nodes;     /* fixed wave size in frontier nodes (positions 5 plies above the
-                                    leaves); 0 = waves sized in time, about 4 ms of device work
+                                    leaves); 0 = waves sized in time, about 2.5 ms of device work
                                     each from the measured rate and leaves per task */
     int use_tt;                  /* pg_tt_mode of the waves; with PG_TT_ON the tables persist
                                     across requests (launcher.h:699-790 keeps its table across runs) */

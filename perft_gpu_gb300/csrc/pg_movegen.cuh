@@ -413,14 +413,14 @@ template <int S> __device__ __forceinline__ KsFacts<S> ks_facts(const Pos& b)
 }
 
 // countMoves / countMovesOutOfCheck (MGB.h:3008-3295, 2825-3002) as one
-// instruction stream for the Kogge-Stone policy.  Check handling is a target
+// instruction stream for the hybrid policy (enemy fills by Kogge-Stone, own
+// sliders by lookup).  Check handling is a target
 // mask: ~own outside check, the check ray (between squares + checker) in
 // single check, nothing in double check; pinned pieces move along their pin
 // line outside check and not at all in check.  The counts are the
 // reference's in every case (proved per term in the comments of the
 // reference-shaped paths above and checked bit-exact by the tests).
-template <int S, bool OWN_BY_LOOKUP = false>
-__device__ __forceinline__ u32 count_from_facts(const Pos& b, const KsFacts<S>& f)
+template <int S> __device__ __forceinline__ u32 count_from_facts(const Pos& b, const KsFacts<S>& f)
 {
     const u64 pawns = f.pawns, occ = f.occ, mine = f.mine, theirs = f.theirs, empty = f.empty;
     const u64 pf = f.pf, pr = f.pr, pd = f.pd, pa = f.pa, pinned = f.pinned, checkers = f.checkers;
@@ -432,50 +432,21 @@ __device__ __forceinline__ u32 count_from_facts(const Pos& b, const KsFacts<S>& 
 
     const u64 my_rq = b.rq & mine, my_bq = b.bq & mine;
     const u64 pin_chk = pinned & chk_all;
-    if constexpr (OWN_BY_LOOKUP) {
-        // pass 2 by table lookup, one per own slider; a pinned piece keeps the
-        // moves along its pin line (none if the line is not its kind)
-        for (u64 s = my_rq & ~pin_chk; s; s &= s - 1) {
-            const int sq = lsb(s);
-            const u64 bit = 1ull << sq;
-            u64 m = SlFancy::rook(sq, b.k | pawns | b.n | b.bq | b.rq) & tgt;
-            if (pinned & bit) m &= (pf & bit) ? file_of(ksq) : (pr & bit) ? rank_of(ksq) : 0ull;
-            n += popc(m);
-        }
-        for (u64 s = my_bq & ~pin_chk; s; s &= s - 1) {
-            const int sq = lsb(s);
-            const u64 bit = 1ull << sq;
-            u64 m = SlFancy::bishop(sq, b.k | pawns | b.n | b.bq | b.rq) & tgt;
-            if (pinned & bit) m &= (pd & bit) ? diag_of(ksq) : (pa & bit) ? anti_of(ksq) : 0ull;
-            n += popc(m);
-        }
-    } else {
-        // pass 2: own slider moves, through the real empty squares (pass 1's
-        // chains treat the king as empty).  The chains are built from an
-        // opaque copy of `empty`, so the compiler builds them here rather than
-        // early, where they would be live across pass 1.
-        u64 empty2 = empty;
-#ifdef __CUDACC__
-        asm volatile("" : "+l"(empty2));
-#endif
-        {
-            const u64 ns = my_rq & ~((pinned ^ pf) | pin_chk);
-            u64 up_att, down_att;
-            vertical_fills(empty2, ns, up_att, down_att);
-            n += popc(up_att & tgt) + popc(down_att & tgt);
-        }
-        {
-            const u64 ew = my_rq & ~((pinned ^ pr) | pin_chk);
-            n += popc(Pro<1, true>(empty2).attacks(ew) & tgt) + popc(Pro<1, false>(empty2).attacks(ew) & tgt);
-        }
-        {
-            const u64 dg = my_bq & ~((pinned ^ pd) | pin_chk);
-            n += popc(Pro<9, true>(empty2).attacks(dg) & tgt) + popc(Pro<9, false>(empty2).attacks(dg) & tgt);
-        }
-        {
-            const u64 ad = my_bq & ~((pinned ^ pa) | pin_chk);
-            n += popc(Pro<7, true>(empty2).attacks(ad) & tgt) + popc(Pro<7, false>(empty2).attacks(ad) & tgt);
-        }
+    // pass 2 by table lookup, one per own slider; a pinned piece keeps the
+    // moves along its pin line (none if the line is not its kind)
+    for (u64 s = my_rq & ~pin_chk; s; s &= s - 1) {
+        const int sq = lsb(s);
+        const u64 bit = 1ull << sq;
+        u64 m = SlFancy::rook(sq, b.k | pawns | b.n | b.bq | b.rq) & tgt;
+        if (pinned & bit) m &= (pf & bit) ? file_of(ksq) : (pr & bit) ? rank_of(ksq) : 0ull;
+        n += popc(m);
+    }
+    for (u64 s = my_bq & ~pin_chk; s; s &= s - 1) {
+        const int sq = lsb(s);
+        const u64 bit = 1ull << sq;
+        u64 m = SlFancy::bishop(sq, b.k | pawns | b.n | b.bq | b.rq) & tgt;
+        if (pinned & bit) m &= (pd & bit) ? diag_of(ksq) : (pa & bit) ? anti_of(ksq) : 0ull;
+        n += popc(m);
     }
 
     for (u64 s = b.n & mine & ~pinned; s; s &= s - 1) n += popc(__ldg(&g_knight[lsb(s)]) & tgt);
@@ -500,10 +471,9 @@ __device__ __forceinline__ u32 count_from_facts(const Pos& b, const KsFacts<S>& 
     return n;
 }
 
-template <int S, bool OWN_BY_LOOKUP = false>
-__device__ __forceinline__ u32 count_moves_ks(const Pos& b)
+template <int S> __device__ __forceinline__ u32 count_moves_ks(const Pos& b)
 {
-    return count_from_facts<S, OWN_BY_LOOKUP>(b, ks_facts<S>(b));
+    return count_from_facts<S>(b, ks_facts<S>(b));
 }
 
 // Rank attacks by subtraction: with file H marked occupied (so that no borrow
@@ -750,7 +720,7 @@ template <int S, class SL>
 __device__ __forceinline__ u32 count_moves(const Pos& b)
 {
     if constexpr (SL::kId == 0) return count_moves_ks1<S>(b);
-    else if constexpr (SL::kId == 3) return count_moves_ks<S, true>(b);
+    else if constexpr (SL::kId == 3) return count_moves_ks<S>(b);
     else return count_moves_mg<S, SL>(b);
 }
 

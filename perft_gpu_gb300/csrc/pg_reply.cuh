@@ -40,15 +40,15 @@
 // The legality rules enter only through the passed count, whose terms are
 // count_moves_ks1's outside check.
 //
-// What bounds it: integer-ALU issue (66-70% busy in this part; the rest is the
-// latency of dependent instructions and table loads with 16 warps an SM), as
-// the count of a made child (about 900 instructions).  The set-wise part costs
-// a node about 5,500, six children's worth, and replaces 71% of its 34 moves,
-// a king recount (about 150) another 9%.
-// Measured (GB300): 4,096 positions at depths 3..6 in 626 ms, 1,237 ms with
-// every child made and counted; one position at depth 7 in 36.2 against 92.5 ms;
-// with every move that is not plain made and counted, and one emission loop
-// per piece, every 16th of those positions took 37.5 ms of leaf time, now 34.9.
+// What bounds it: integer-ALU issue (78-79% busy over the leaf; the rest is the
+// latency of dependent instructions and table loads with 16 warps an SM, and
+// loops over a node's pieces of different length in a warp's lanes), as the
+// count of a made child (about 900 instructions).  Of a node's 34 moves 73% are
+// counted in sets, 10.3% are a king recount (about 150 instructions), 16.9% are
+// made; every 16th of 4,096 positions at depths 3..6 spends 16.7 ms of leaf time
+// here, 10.7 on made children, 3.1 on king recounts.
+// Measured (GB300): those 4,096 positions in 519 ms, 1,203 ms with every child
+// made and counted; one position at depth 7 in 29.3 against 92.5 ms of leaf time.
 #pragma once
 #include "pg_movegen.cuh"
 
