@@ -1534,6 +1534,17 @@ int pg_perft_batch_device(const pg_board* d_pos, const uint8_t* d_depths, uint32
     return end_call(opts);
 }
 
+// A call that fails between its launches still has kernels (or a copy) reading
+// the pinned inputs: it waits for them before it returns, since the next call
+// writes its own inputs there.
+struct PinnedInputs {
+    bool in_use = false;
+    ~PinnedInputs()
+    {
+        if (in_use) cudaStreamSynchronize(engine().stream);
+    }
+};
+
 int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint64_t* out, const pg_opts* opts)
 {
     if (!pos || !depths || !out) { set_error("null argument"); return PG_ERR_INVALID_ARGUMENT; }
@@ -1555,9 +1566,11 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     u64* d_out = (u64*)(s + pb + db);
     PG_TRY(begin_call(opts));
     RootInfo info{0, 15, 0, true};
+    PinnedInputs pinned;
     if (small) {
         memcpy(E.host_io, pos, pb);
         memcpy(E.host_io + pb, depths, n);
+        pinned.in_use = true;
         for (u32 i = 0; i < n; i++) {
             info.white += !(pos[i].pawns >> 63);
             info.mind = std::min<u32>(info.mind, depths[i]);
@@ -1596,6 +1609,7 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
             PG_CUDA(cudaMemcpyAsync(h_out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
             PG_TRY(end_call(nullptr));
         }
+        pinned.in_use = false;  // waited for
         memcpy(out, h_out, ob);
     } else {
         PG_CUDA(cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, E.stream));
@@ -1628,6 +1642,7 @@ int pg_perft_divide(const pg_board* pos, int depth, pg_move* moves, uint64_t* co
     {
         Engine& E = engine();
         std::lock_guard<std::mutex> lk(E.mu);
+        PG_TRY(check_ready());
         Pos* d = (Pos*)E.host_io;
         u16* dm = (u16*)(E.host_io + 256 * 48);
         for (u32 i = 0; i < *n; i++) memcpy(d + i, pos, sizeof(Pos));
