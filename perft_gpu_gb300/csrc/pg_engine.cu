@@ -358,7 +358,7 @@ static int run_children(const Variant& v, int L, u32 start, u32 n, int side, int
 // than AHEAD_MOVES a node, on boards of no game) stops the sequence on the
 // device; ahead_failed() tells afterwards, and the caller runs the whole call
 // level by level.  One position at depth 3 / 4 / 5: 66 / 93 / 126 us waiting at
-// each level, 60 / 81 / 114 us so.
+// each level, 60 / 81 / 114 us so, and k_step takes a launch off each first level.
 static int run_ahead(const Variant& v, u32 start, u32 n, int side0, int minrem, int maxrem, u64* acc)
 {
     Engine& E = engine();
@@ -374,11 +374,18 @@ static int run_ahead(const Variant& v, u32 start, u32 n, int side0, int minrem, 
             return run_children(v, L, start, n, side, minrem, maxrem, acc, n_dev);
         PG_TRY(ensure_level(L + 1, n * AHEAD_MOVES));
         const Ahead ahead{n_dev, E.ahead_n + E.ahead_plans};
+        PlanOut* plan = E.plan_host + 1 + E.ahead_plans;
         PG_TICKET(done);
-        PG_CUDA(ops_for(v.slider).count_plan(side, lb.v, start, n, lb.cnt, (u32)lp + 1, lb.offs, E.lv[L + 1].cap,
-                                             E.plan_host + 1 + E.ahead_plans, done, E.err, ahead, E.stream));
-        E.st.launches++;
-        PG_TRY(launch_expand(v, side, lb.v, start, 0, n, lb.offs, E.lv[L + 1].v, ahead));
+        if (n <= (n_dev ? AHEAD_MOVES : STEP_MAX)) {
+            PG_CUDA(ops_for(v.slider).step(side, lb.v, start, n, lb.cnt, (u32)lp + 1, lb.offs, E.lv[L + 1].cap, plan, E.err, ahead,
+                                           E.lv[L + 1].v, done, E.stream));
+            E.st.launches++;
+        } else {
+            PG_CUDA(ops_for(v.slider).count_plan(side, lb.v, start, n, lb.cnt, (u32)lp + 1, lb.offs, E.lv[L + 1].cap, plan, done,
+                                                 E.err, ahead, E.stream));
+            E.st.launches++;
+            PG_TRY(launch_expand(v, side, lb.v, start, 0, n, lb.offs, E.lv[L + 1].v, ahead));
+        }
         E.ahead_plans++;
         n_dev = ahead.children;
         n *= AHEAD_MOVES;

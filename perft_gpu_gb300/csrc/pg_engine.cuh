@@ -22,6 +22,11 @@ constexpr u32 PLAN_FUSED_MAX = 8192;  // nodes of a level whose counts, scan and
 // children a node, the most a position of a game has, fit the smallest level buffer
 constexpr u32 AHEAD_MOVES = 218;
 constexpr u32 AHEAD_NODES = 1u << 16;
+// Roots of a level that one CTA counts and expands (k_step); below one root the
+// level it makes is small enough whatever the position.  Depth 3 of 4 / 16 / 32 /
+// 64 / 256 roots: 67 / 69 / 70 / 75 / 90 us so, 70 / 70 / 70 / 73 / 75 with a count
+// and an expansion over the device.
+constexpr u32 STEP_MAX = 24;
 constexpr int AHEAD_PLANS = 4;  // two levels for each side of the roots (1 x 218 x 218 is under AHEAD_NODES)
 constexpr u32 HOST_IO_ROOTS = 4096;   // largest host-array call staged in pinned memory and checked on the host
 constexpr u32 HOST_IO_BYTES = HOST_IO_ROOTS * (48 + 1 + 8) + 64;

@@ -320,30 +320,17 @@ __global__ void k_count_level(LevelView lv, u32 start, u32 n, u32* __restrict__ 
     count_level_body<S, SL>(lv, start, n, cnt, min_rem);
 }
 
-// Children counts, their scan and the chunk plan of a small level (n up to
-// PLAN_FUSED_MAX) in one launch: the last CTA to finish its counts scans them
-// all.  The plan goes straight to pinned host memory (nchunks 0: the children do
-// not fit one chunk of `cap`, k_plan has to split them; pad: the error bits).
-// ahead: the level's size (null: n) and where its children's number goes for a
-// launch sequence that does not return to the host between levels; 0 there when
-// they do not fit, so that the launches behind do nothing.
-template <int S, class SL>
-__global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
-                                                    PlanOut* plan, u32* done, const u32* err, Ahead ahead)
+// The scan of a small level's children counts and its chunk plan, by one CTA of
+// 256; returns the number of children.  The plan goes straight to pinned host
+// memory (nchunks 0: the children do not fit one chunk of `cap`, k_plan has to
+// split them; pad: the error bits).  children (or null): their number for a launch
+// sequence that does not return to the host between levels; 0 there when they do
+// not fit, so that the launches behind do nothing.
+__device__ __forceinline__ u64 plan_level(u32 n, const u32* cnt, u64* offs, u64 cap, PlanOut* plan, const u32* err, u32* children)
 {
-    stage_tables<SL>();
-    if (ahead.nodes) n = *ahead.nodes;
-    count_level_body<S, SL>(lv, start, n, cnt, min_rem);
     constexpr int T = 256;
-    __shared__ u32 s_done;
     __shared__ u64 s_warp[T / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_done = atomicAdd(done, 1u);
-    __syncthreads();
-    if (s_done != gridDim.x - 1) return;
-    __threadfence();
     const u32 per = (n + T - 1) / T, c0 = min(n, tid * per), c1 = min(n, c0 + per);
     u64 sum = 0;
     for (u32 i = c0; i < c1; i++) sum += __ldcg(cnt + i);
@@ -367,7 +354,7 @@ __global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32
     if (tid == 0) {
         offs[n] = total;
         plan->nchunks = total <= cap ? 1u : 0u;
-        if (ahead.children) *ahead.children = total <= cap ? (u32)total : 0u;
+        if (children) *children = total <= cap ? (u32)total : 0u;
         plan->pad = *err;
         plan->total = total;
         plan->bnd[0] = 0;
@@ -375,6 +362,27 @@ __global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32
         plan->coff[0] = 0;
         plan->coff[1] = total;
     }
+    return total;
+}
+
+// Children counts, their scan and the chunk plan of a small level (n up to
+// PLAN_FUSED_MAX) in one launch: the last CTA to finish its counts scans them
+// all.  ahead: the level's size (null: n) and where its children's number goes.
+template <int S, class SL>
+__global__ void __launch_bounds__(256) k_count_plan(LevelView lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
+                                                    PlanOut* plan, u32* done, const u32* err, Ahead ahead)
+{
+    stage_tables<SL>();
+    if (ahead.nodes) n = *ahead.nodes;
+    count_level_body<S, SL>(lv, start, n, cnt, min_rem);
+    __shared__ u32 s_done;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_done = atomicAdd(done, 1u);
+    __syncthreads();
+    if (s_done != gridDim.x - 1) return;
+    __threadfence();
+    plan_level(n, cnt, offs, cap, plan, err, ahead.children);
 }
 
 constexpr int LEAF_GATHER = 4;  // nodes a thread looks at when the CTA collects the live ones of a sparse level
@@ -526,6 +534,25 @@ __global__ void __launch_bounds__(T, min_blocks<T>()) k_expand(LevelView in, u32
         if (ahead.nodes) b = *ahead.nodes;
     }
     expand_body<S, SL, T, QCAP>(in, start, a, b, offs, out, ticket, parent_out, whole_grid());
+}
+
+// Counts, plan and expansion of a level of a few nodes (STEP_MAX) by one CTA of
+// 256 threads.  Such a call is a chain of launches, each as long as a thread takes
+// through its code: one less a level.  One position at depth 3 / 4 / 5: 61 / 82 /
+// 121 -> 56 / 73 / 111 us (means of three).
+template <int S, class SL, int QCAP>
+__global__ void __launch_bounds__(256, min_blocks<256>()) k_step(LevelView in, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs,
+                                                                u64 cap, PlanOut* plan, const u32* err, Ahead ahead, LevelView out,
+                                                                u32* ticket)
+{
+    stage_tables<SL>();
+    if (ahead.nodes) n = *ahead.nodes;
+    count_level_body<S, SL>(in, start, n, cnt, min_rem);
+    __syncthreads();
+    const u64 total = plan_level(n, cnt, offs, cap, plan, err, ahead.children);
+    __syncthreads();
+    if (total == 0 || total > cap) return;
+    expand_body<S, SL, 256, QCAP>(in, start, 0, n, offs, out, ticket, nullptr, Share{0u, 1u});
 }
 
 }  // namespace pg

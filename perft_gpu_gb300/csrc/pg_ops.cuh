@@ -21,6 +21,8 @@ struct SliderOps {
                                cudaStream_t st, int num_sms);
     cudaError_t (*count_plan)(int side, const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap,
                               PlanOut* plan, u32* done, const u32* err, Ahead ahead, cudaStream_t st);
+    cudaError_t (*step)(int side, const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap, PlanOut* plan,
+                        const u32* err, Ahead ahead, const LevelView& out, u32* ticket, cudaStream_t st);
     cudaError_t (*count_batch)(const Pos* in, u32 n, u32* out, cudaStream_t st);
     cudaError_t (*gen_moves_batch)(const Pos* in, u32 n, u16* out, u32* nout, cudaStream_t st);
     cudaError_t (*gen_boards_batch)(const Pos* in, u32 n, Pos* out, u32* nout, cudaStream_t st);

@@ -148,6 +148,27 @@ cudaError_t count_plan_any(int side, const LevelView& lv, u32 start, u32 n, u32*
                 : count_plan_t<0, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, ahead, st);
 }
 
+template <int S, class SL>
+cudaError_t step_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap, PlanOut* plan, const u32* err,
+                   Ahead ahead, const LevelView& out, u32* ticket, cudaStream_t st)
+{
+    constexpr int Q = QcapFor<SL, 256>::expand;
+    using L = BlockSmem<SL, 256, Q>;
+    auto fn = k_step<S, SL, Q>;
+    static cudaError_t attr = set_smem(fn, L::bytes);
+    if (attr) return attr;
+    fn<<<1, 256, L::bytes, st>>>(lv, start, n, cnt, min_rem, offs, cap, plan, err, ahead, out, ticket);
+    return cudaGetLastError();
+}
+
+template <class SL>
+cudaError_t step_any(int side, const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem, u64* offs, u64 cap, PlanOut* plan,
+                     const u32* err, Ahead ahead, const LevelView& out, u32* ticket, cudaStream_t st)
+{
+    return side ? step_t<1, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, err, ahead, out, ticket, st)
+                : step_t<0, SL>(lv, start, n, cnt, min_rem, offs, cap, plan, err, ahead, out, ticket, st);
+}
+
 inline int small_grid(u32 n, int T) { return (int)std::max<u32>(1, std::min<u32>((n + T - 1) / T, 8192)); }
 
 template <class SL>
@@ -203,7 +224,7 @@ cudaError_t playouts(const Pos& start, u64 seed, u32 n, int min_plies, int max_p
 #define PG_DEFINE_OPS(SLT, NAME, ENUM)                                                                   \
     const SliderOps g_ops_##NAME = {#NAME,          ENUM,                    upload_tables<SLT>,           \
                                     leaf_any<SLT>,  expand_any<SLT>,         count_level_any<SLT>,         \
-                                    count_plan_any<SLT>,                                                          \
+                                    count_plan_any<SLT>, step_any<SLT>,                                           \
                                     count_batch<SLT>, gen_moves_batch<SLT>,  gen_boards_batch<SLT>,        \
                                     make_batch,     playouts<SLT>};
 

@@ -162,3 +162,14 @@ def test_duplicates_within_and_across_depths(pg, orc, lo, hi):
         pg.tt_clear()
         assert np.array_equal(pg.perft_batch(boards, depths, use_tt=mode, tt_bytes=1 << 28), want)
     pg.tt_clear()
+
+
+@pytest.mark.parametrize("n", [1, 23, 24, 25])
+def test_one_cta_steps_a_small_level(pg, orc, n):
+    """Up to 24 roots, and the children of one, are counted and expanded by one
+    CTA: its queue has more than one window on boards with many moves."""
+    for fen in (MANY, SHARP):
+        depth = 4 if n == 1 else 3
+        got = pg.perft_batch(_copies(pg, fen, n), np.full(n, depth, np.uint8), slider="byte")
+        assert np.array_equal(got, pg.perft_batch(_copies(pg, fen, n), np.full(n, depth, np.uint8), slider="ks"))
+        assert (got == orc.perft(orc.fen(fen), depth)).all()
