@@ -8,6 +8,8 @@
 //                   bounded spin (replaces moderngpu ScanD, scan.cuh:330)
 //   k_plan          greedy split of a level into chunks whose children fit
 //                   the next level's buffer (HBM budget)
+//   k_count_plan    the three in one launch for a small level; k_step: with
+//                   the expansion as well, for a few nodes
 //   k_expand        generate + make into the next level; the CTA stages its
 //                   nodes in shared memory, emits (parent, move) entries into
 //                   a shared queue and writes children coalesced in 16-byte
