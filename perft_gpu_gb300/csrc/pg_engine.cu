@@ -698,11 +698,13 @@ static int device_max_depth(const unsigned char* d_depths, u32 n, int* maxd);
 // launch) stays valid for any contents of the same buffers, size and largest
 // depth (the level buffers are prepared for it); only the largest depth is
 // read back per call.
-static int perft_batch_graph_persistent(const Pos* d_pos, const unsigned char* d_depths, u32 n, u64* d_out)
+// maxd: the largest depth when the caller knows it (else -1: a kernel, a copy and
+// a wait; one position at depth 3 took 109 us with them, two more clears and the
+// timing events, 75 without)
+static int perft_batch_graph_persistent(const Pos* d_pos, const unsigned char* d_depths, u32 n, u64* d_out, int maxd = -1)
 {
     Engine& E = engine();
-    int maxd = 0;
-    PG_TRY(device_max_depth(d_depths, n, &maxd));
+    if (maxd < 0) PG_TRY(device_max_depth(d_depths, n, &maxd));
     if (maxd > 15) {
         set_error("depth %d out of range 0..15", maxd);
         return PG_ERR_INVALID_ARGUMENT;
@@ -743,15 +745,17 @@ static int perft_batch_graph_persistent(const Pos* d_pos, const unsigned char* d
     } else {
         E.st.graph_replays = 1;
     }
-    cudaEventRecord(E.ev0, E.stream);
+    if (E.timing) cudaEventRecord(E.ev0, E.stream);
     PG_CUDA(cudaGraphLaunch(g.exec, E.stream));
-    cudaEventRecord(E.ev1, E.stream);
-    PG_CUDA(cudaEventSynchronize(E.ev1));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, E.ev0, E.ev1);
-    E.st.device_ms = ms;
-    E.st.leaf_kernel_ms = ms;
     E.st.launches = 1;
+    if (E.timing) {
+        cudaEventRecord(E.ev1, E.stream);
+        PG_CUDA(cudaEventSynchronize(E.ev1));
+        float ms = 0;
+        cudaEventElapsedTime(&ms, E.ev0, E.ev1);
+        E.st.device_ms = ms;
+        E.st.leaf_kernel_ms = ms;
+    }
     return PG_OK;
 }
 
@@ -925,9 +929,8 @@ int perft_core_persistent(const Pos* d_pos, const unsigned char* d_depths, const
     A.groups = d_groups;
     A.n = n;
     A.acc = acc;
-    if (zero_acc) PG_CUDA(cudaMemsetAsync(acc, 0, (u64)n * sizeof(u64), E.stream));
+    A.zero_acc = zero_acc;  // by the launch, in its partition phase
     PG_CUDA(cudaMemsetAsync(E.persist_ctl, 0, sizeof(PersistCtl), E.stream));
-    PG_CUDA(cudaMemsetAsync(&E.persist_ctl->part[2], 0xFF, sizeof(u32), E.stream));
     PG_CUDA(cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream));
     const bool timed = E.plan_mode != PLAN_REPLAY && E.timing;
     if (timed) cudaEventRecord(E.ev0, E.stream);
@@ -1614,7 +1617,7 @@ int pg_perft_batch(const pg_board* pos, const uint8_t* depths, uint32_t n, uint6
     if (opts && opts->use_tt) {
         PG_TRY(tt_perft_batch_device(d_pos, d_dep, n, d_out, opts));
     } else if (opts && opts->graph && opts->persistent) {
-        PG_TRY(perft_batch_graph_persistent(d_pos, d_dep, n, d_out));
+        PG_TRY(perft_batch_graph_persistent(d_pos, d_dep, n, d_out, (int)info.maxd));
     } else if (opts && opts->graph) {
         PG_TRY(perft_batch_graph_locked(d_pos, d_dep, n, d_out, opts));
     } else {

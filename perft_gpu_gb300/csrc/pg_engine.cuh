@@ -78,9 +78,9 @@ struct PlanOut {
 enum PlanMode { PLAN_NONE = 0, PLAN_RECORD = 1, PLAN_REPLAY = 2 };
 
 // control words of one persistent launch (pg_persist.cuh; device memory,
-// zeroed by the host before the launch, part[2] = 0xFFFFFFFF): grid barrier
-// arrival count and generation, abort flag, root partition counters (white,
-// black, min depth, max depth)
+// zeroed by the host before the launch): grid barrier arrival count and
+// generation, abort flag, root partition counters (white, black, the complement of
+// the min depth, max depth)
 struct PersistCtl {
     u32 bar_count, bar_gen, abort, pad;
     u32 part[4];
@@ -95,6 +95,7 @@ struct PersistArgs {
     const u32* groups;  // group id per root (null: the root's index)
     u32 n;
     u64* acc;  // per-group counts (added to)
+    u32 zero_acc;  // the first n of them start at 0
     LevelView lv[MAX_LEVELS];
     u32* cnt[MAX_LEVELS];
     u64* offs[MAX_LEVELS];

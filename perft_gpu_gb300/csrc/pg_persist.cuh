@@ -257,13 +257,14 @@ __global__ void __launch_bounds__(PERSIST_T, min_blocks<PERSIST_T>()) k_persist(
         store_board(A.lv[0], slot, b);
         A.lv[0].grp[slot] = A.groups ? A.groups[i] : i;
         A.lv[0].rem[slot] = (unsigned char)d;
-        atomicMin(&ctl->part[2], d);
+        if (A.zero_acc) A.acc[i] = 0;
+        atomicMax(&ctl->part[2], ~d);
         atomicMax(&ctl->part[3], d);
     }
     if (!grid_barrier(ctl, A.err)) return;
     using ARef = cuda::atomic_ref<u32, cuda::thread_scope_device>;
     const u32 nw = ARef(ctl->part[0]).load(cuda::memory_order_relaxed);
-    const int mind = (int)ARef(ctl->part[2]).load(cuda::memory_order_relaxed);
+    const int mind = (int)~ARef(ctl->part[2]).load(cuda::memory_order_relaxed);
     const int maxd = (int)ARef(ctl->part[3]).load(cuda::memory_order_relaxed);
     if (maxd > 15) {
         if (blockIdx.x == 0 && threadIdx.x == 0) persist_fail(A, ERR_PLAN_OVERFLOW);
