@@ -1662,21 +1662,32 @@ int pg_perft_divide(const pg_board* pos, int depth, pg_move* moves, uint64_t* co
         set_error("bad argument");
         return PG_ERR_INVALID_ARGUMENT;
     }
-    PG_TRY(pg_generate_moves(pos, moves, n));
-    if (*n == 0) return PG_OK;
     pg_board kids[256];
     {
+        // the moves and the children they make, without a wait between: in pinned
+        // memory, as op_batch does for one position (depth 6: 757 -> 747 us)
         Engine& E = engine();
         std::lock_guard<std::mutex> lk(E.mu);
         PG_TRY(check_ready());
-        Pos* d = (Pos*)E.host_io;
-        u16* dm = (u16*)(E.host_io + 256 * 48);
-        for (u32 i = 0; i < *n; i++) memcpy(d + i, pos, sizeof(Pos));
-        memcpy(dm, moves, *n * 2);
-        PG_CUDA(g_ops_ks.make_batch(d, dm, *n, E.stream));
+        if (!valid_board(*pos)) { set_error("not a valid board"); return PG_ERR_INVALID_POSITION; }
+        Pos* root = (Pos*)E.host_io;
+        u16* mv = (u16*)(E.host_io + 64);
+        u32* cnt = (u32*)(E.host_io + 64 + 512);
+        Pos* out = (Pos*)(E.host_io + 64 + 512 + 64);
+        memcpy(root, pos, sizeof(Pos));
+        PinnedInputs pinned;
+        pinned.in_use = true;
+        const SliderOps& ops = ops_for(slider_of(PG_SLIDER_AUTO));
+        PG_CUDA(ops.gen_moves_batch(root, 1, mv, cnt, E.stream));
+        PG_CUDA(ops.make_children(root, mv, cnt, out, E.stream));
         PG_CUDA(cudaStreamSynchronize(E.stream));
-        memcpy(kids, d, *n * 48);
+        pinned.in_use = false;
+        *n = *cnt;
+        memcpy(moves, mv, 512);
+        if (*n > 256) { set_error("more than 256 moves"); return PG_ERR_CAPACITY; }
+        memcpy(kids, out, *n * sizeof(Pos));
     }
+    if (*n == 0) return PG_OK;
     uint8_t dep[256];
     for (u32 i = 0; i < *n; i++) dep[i] = (uint8_t)(depth - 1);
     return pg_perft_batch(kids, dep, *n, counts, opts);

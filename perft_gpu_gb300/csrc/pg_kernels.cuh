@@ -252,6 +252,17 @@ static __global__ void k_make_batch(Pos* __restrict__ pos, const u16* __restrict
     }
 }
 
+// the children of one position by its *n moves (at most 256)
+static __global__ void k_make_children(const Pos* __restrict__ root, const u16* __restrict__ mv, const u32* __restrict__ n,
+                                       Pos* __restrict__ out)
+{
+    const u32 i = threadIdx.x;
+    if (i >= min(*n, 256u)) return;
+    Pos b = *root;
+    if (st_side(b)) make_move<1>(b, mv[i]); else make_move<0>(b, mv[i]);
+    out[i] = b;
+}
+
 __device__ __forceinline__ u64 splitmix_next(u64& s)
 {
     u64 z = (s += 0x9E3779B97F4A7C15ull);

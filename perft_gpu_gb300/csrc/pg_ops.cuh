@@ -27,6 +27,7 @@ struct SliderOps {
     cudaError_t (*gen_moves_batch)(const Pos* in, u32 n, u16* out, u32* nout, cudaStream_t st);
     cudaError_t (*gen_boards_batch)(const Pos* in, u32 n, Pos* out, u32* nout, cudaStream_t st);
     cudaError_t (*make_batch)(Pos* pos, const u16* mv, u32 n, cudaStream_t st);
+    cudaError_t (*make_children)(const Pos* root, const u16* mv, const u32* n, Pos* out, cudaStream_t st);
     cudaError_t (*playouts)(const Pos& start, u64 seed, u32 n, int min_plies, int max_plies, int min_moves,
                             int depth_lo, int depth_hi, Pos* out, unsigned char* depths, u32* err, cudaStream_t st);
 };

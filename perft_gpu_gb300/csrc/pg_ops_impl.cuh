@@ -207,6 +207,12 @@ inline cudaError_t make_batch(Pos* pos, const u16* mv, u32 n, cudaStream_t st)
     return cudaGetLastError();
 }
 
+inline cudaError_t make_children(const Pos* root, const u16* mv, const u32* n, Pos* out, cudaStream_t st)
+{
+    k_make_children<<<1, 256, 0, st>>>(root, mv, n, out);
+    return cudaGetLastError();
+}
+
 template <class SL>
 cudaError_t playouts(const Pos& start, u64 seed, u32 n, int min_plies, int max_plies, int min_moves, int depth_lo,
                      int depth_hi, Pos* out, unsigned char* depths, u32* err, cudaStream_t st)
@@ -226,6 +232,6 @@ cudaError_t playouts(const Pos& start, u64 seed, u32 n, int min_plies, int max_p
                                     leaf_any<SLT>,  expand_any<SLT>,         count_level_any<SLT>,         \
                                     count_plan_any<SLT>, step_any<SLT>,                                           \
                                     count_batch<SLT>, gen_moves_batch<SLT>,  gen_boards_batch<SLT>,        \
-                                    make_batch,     playouts<SLT>};
+                                    make_batch,     make_children,           playouts<SLT>};
 
 }  // namespace pg
