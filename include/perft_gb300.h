@@ -238,7 +238,8 @@ int pg_perft_split(const pg_board *pos, int depth, int split_plies, pg_move *mov
  * PG_ERR_DEVICE_TIMEOUT, with the context still usable.
  * PG_SELFTEST_FAIL_NEXT_ALLOC makes the next level allocation fail on the
  * host, so the following call returns PG_ERR_OUT_OF_MEMORY and the one after
- * it works.  No counterpart in the reference. */
+ * it works; with k << 8 added, k level allocations succeed before the one that
+ * fails.  No counterpart in the reference. */
 enum { PG_SELFTEST_BOUNDED_WAIT = 1, PG_SELFTEST_FAIL_NEXT_ALLOC = 2 };
 int pg_selftest(int which);
 

@@ -174,8 +174,8 @@ int ensure_level(int L, u64 need)
     }
     const u64 bytes = cap * 48 + cap * 4 + cap + 16 + cap * 4 + (cap + 1) * 8 + 256;
     void* blk = nullptr;
-    cudaError_t e = E.fail_next_alloc ? cudaErrorMemoryAllocation : cudaMalloc(&blk, bytes);
-    E.fail_next_alloc = false;
+    const bool refuse = E.fail_alloc_in && --E.fail_alloc_in == 0;
+    cudaError_t e = refuse ? cudaErrorMemoryAllocation : cudaMalloc(&blk, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error("level %d buffer of %llu nodes (%llu bytes) failed: %s", L, (unsigned long long)cap,
@@ -405,6 +405,27 @@ static bool ahead_failed()
     return false;
 }
 
+// What the tuner's own calls change and the call that it runs inside goes on
+// with, put back on every way out: the stats, the timing switch, and the
+// counters and error bits of a call's start (begin_call).  The partition
+// counters are among those: perft_core with known roots places them from zero
+// without a clear of its own, also when the tuner gave up half-way.
+struct TunerScope {
+    const pg_stats st = engine().st;
+    const bool timing = engine().timing;
+    void* buf = nullptr;  // the calibration batch
+    ~TunerScope()
+    {
+        Engine& E = engine();
+        if (buf) cudaFree(buf);
+        E.st = st;
+        E.timing = timing;
+        E.leaf_ev_used = 0;
+        E.ticket_next = 0;
+        cudaMemsetAsync(E.tickets, 0, (MAX_TICKETS + 1) * sizeof(u32), E.stream);
+    }
+};
+
 // The autotuner: per root depth 3..6, a seeded calibration batch is timed
 // with each candidate leaf variant (slider policy x CTA size); the fastest
 // serves that depth (shallower depths take depth 3's, deeper ones depth 6's).
@@ -416,8 +437,7 @@ static int autotune_locked()
     Engine& E = engine();
     if (E.tuned) return PG_OK;
     const auto t0 = std::chrono::steady_clock::now();
-    const pg_stats saved = E.st;
-    const bool timing = E.timing;
+    TunerScope scope;
     E.timing = true;
     struct Cal {
         int depth;
@@ -429,10 +449,9 @@ static int autotune_locked()
                            {PG_SLIDER_HYBRID, 256},       {PG_SLIDER_HYBRID, 512}};
     const int ncand = (int)(sizeof(cand) / sizeof(cand[0]));
     const u32 nmax = 2048;
-    void* buf = nullptr;
-    PG_CUDA(cudaMalloc(&buf, nmax * (48 + 1 + 8) + 256));
-    Pos* d_pos = (Pos*)buf;
-    unsigned char* d_dep = (unsigned char*)buf + nmax * 48;
+    PG_CUDA(cudaMalloc(&scope.buf, nmax * (48 + 1 + 8) + 256));
+    Pos* d_pos = (Pos*)scope.buf;
+    unsigned char* d_dep = (unsigned char*)scope.buf + nmax * 48;
     u64* d_out = (u64*)(((uintptr_t)(d_dep + nmax) + 15) & ~(uintptr_t)15);
     pg_board start;
     pg_board_from_fen("rnbqkbnr/pppppppp/8/8/8/8/PPPPPPPP/RNBQKBNR w KQkq - 0 1", &start);
@@ -483,11 +502,7 @@ static int autotune_locked()
             E.tuned_leaf_plies = ms1 < best_ms ? 1 : 2;
         }
     }
-    cudaFree(buf);
-    E.timing = timing;
     if (rc != PG_OK) return rc;
-    E.ticket_next = 0;  // the counters as it found them
-    PG_CUDA(cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream));
     for (int d = 0; d < 3; d++) {
         E.tuned_slider[d] = E.tuned_slider[3];
         E.tuned_T[d] = E.tuned_T[3];
@@ -496,7 +511,6 @@ static int autotune_locked()
         E.tuned_slider[d] = E.tuned_slider[6];
         E.tuned_T[d] = E.tuned_T[6];
     }
-    E.st = saved;
     E.tuned = true;
     E.tune_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return PG_OK;
@@ -1501,8 +1515,8 @@ int pg_selftest(int which)
     std::lock_guard<std::mutex> lk(E.mu);
     PG_TRY(check_ready());
     if (which == PG_SELFTEST_BOUNDED_WAIT) return selftest_bounded_wait();
-    if (which == PG_SELFTEST_FAIL_NEXT_ALLOC) {
-        E.fail_next_alloc = true;
+    if (which > 0 && (which & 0xFF) == PG_SELFTEST_FAIL_NEXT_ALLOC) {
+        E.fail_alloc_in = 1u + (u32)(which >> 8);
         // drop the level buffers so that the next call must allocate
         cudaStreamSynchronize(E.stream);
         E.alloc_gen++;

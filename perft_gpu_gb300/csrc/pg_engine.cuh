@@ -190,8 +190,8 @@ struct Engine {
     int tuned_T[16] = {};
     double tuned_rate[16] = {};
     double tune_seconds = 0;
-    // host-side fault injection for tests: the next level allocation fails
-    bool fail_next_alloc = false;
+    // host-side fault injection for tests: which of the next level allocations fails (0: none)
+    u32 fail_alloc_in = 0;
 };
 
 Engine& engine();
