@@ -1330,6 +1330,7 @@ int pg_init(const pg_config* cfg)
     Engine& E = engine();
     std::lock_guard<std::mutex> lk(E.mu);
     if (E.ready) return PG_OK;
+    E.generation++;
     const int rc = init_locked(E, cfg);
     if (rc != PG_OK) release_engine(E);  // a later pg_init starts clean
     return rc;

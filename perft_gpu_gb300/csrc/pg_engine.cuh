@@ -109,7 +109,7 @@ struct PersistArgs {
     u32* err;
 };
 // the persistent launch (Kogge-Stone translation unit); *grid = CTAs launched.
-// persist_setup allows the kernel its shared memory (once, outside a capture).
+// persist_setup makes the kernel ready to be launched (outside a capture).
 cudaError_t persist_setup();
 cudaError_t persist_launch(const PersistArgs& a, cudaStream_t st, int num_sms, int* grid);
 // threads per CTA of the persistent launch: two CTAs of 256 an SM.  The leaf
@@ -138,6 +138,7 @@ struct GraphCache {
 struct Engine {
     std::mutex mu;
     bool ready = false;
+    u32 generation = 0;  // which pg_init of the process this is, from 1 on
     int device = 0;
     int num_sms = 0;
     int verbose = 0;
@@ -195,6 +196,28 @@ struct Engine {
 };
 
 Engine& engine();
+
+// What one kernel needs before its first launch: dynamic shared memory above
+// 48 KB, and how many CTAs an SM holds, which its grids are made of.  Both belong
+// to the device's context, so they are asked for again after every pg_init: the
+// engine may be on another device then, or behind a device reset.  One static of
+// it a launch wrapper, used with the engine's lock held.
+struct KernelSetup {
+    u32 generation = 0;
+    int per_sm = 0;
+    cudaError_t once(const void* fn, int threads, int smem)
+    {
+        if (generation == engine().generation) return cudaSuccess;
+        cudaError_t e = cudaSuccess;
+        if (smem > 48 * 1024) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+        if (e == cudaSuccess && per_sm < 1) e = cudaErrorLaunchOutOfResources;
+        if (e == cudaSuccess) generation = engine().generation;
+        else cudaGetLastError();
+        return e;
+    }
+};
+
 void set_error(const char* fmt, ...);
 
 // engine internals shared by the translation units (call with engine().mu held)

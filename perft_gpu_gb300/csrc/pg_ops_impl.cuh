@@ -22,16 +22,6 @@ template <class SL, int T> struct QcapFor {
     static constexpr int expand = SL::kId == 2 ? T * 8 : T * 64;
 };
 
-// CTAs of a kernel an SM holds (each launch wrapper asks once)
-inline int resident_ctas(const void* fn, int T, int smem)
-{
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, smem) != cudaSuccess || per_sm < 1) {
-        cudaGetLastError();
-        per_sm = 1;
-    }
-    return per_sm;
-}
 inline int full_grid(int per_sm, int T, u64 items, int num_sms)
 {
     const u64 want = std::max<u64>(1, (items + T - 1) / T);
@@ -44,12 +34,6 @@ cudaError_t upload_tables(const HostTables& t)
     return upload_static_tables(t);
 }
 
-template <class K> cudaError_t set_smem(K fn, int bytes)
-{
-    return bytes > 48 * 1024 ? cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)
-                             : cudaSuccess;
-}
-
 template <int S, class SL, int T, bool SPARSE>
 cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket, u32 max_rem, const u32* n_dev,
                    cudaStream_t st, int sms)
@@ -57,11 +41,10 @@ cudaError_t leaf_t(const LevelView& lv, u32 start, u32 n, u64* acc, u32* ticket,
     constexpr int Q = QcapFor<SL, T>::leaf;
     using L = LeafSmem<SL, T, Q>;
     auto fn = k_leaf<S, SL, T, Q, SPARSE>;
-    static cudaError_t attr = set_smem(fn, L::bytes);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)fn, T, L::bytes)) return e;
     // a CTA for every node until the chip is full (node_chunk)
-    static const int per_sm = resident_ctas((const void*)fn, T, L::bytes);
-    const int grid = full_grid(per_sm, T, SPARSE ? n : (u64)n * T, sms);
+    const int grid = full_grid(setup.per_sm, T, SPARSE ? n : (u64)n * T, sms);
     fn<<<grid, T, L::bytes, st>>>(lv, start, n, acc, ticket, max_rem, n_dev);
     return cudaGetLastError();
 }
@@ -73,10 +56,9 @@ cudaError_t expand_t(const LevelView& in, u32 start, u32 a, u32 b, const u64* of
     constexpr int Q = QcapFor<SL, T>::expand;
     using L = BlockSmem<SL, T, Q>;
     auto fn = k_expand<S, SL, T, Q>;
-    static cudaError_t attr = set_smem(fn, L::bytes);
-    if (attr) return attr;
-    static const int per_sm = resident_ctas((const void*)fn, T, L::bytes);
-    const int grid = full_grid(per_sm, T, (u64)(b - a) * T, sms);
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)fn, T, L::bytes)) return e;
+    const int grid = full_grid(setup.per_sm, T, (u64)(b - a) * T, sms);
     fn<<<grid, T, L::bytes, st>>>(in, start, a, b, offs, out, ticket, nullptr, ahead);
     return cudaGetLastError();
 }
@@ -112,10 +94,9 @@ cudaError_t count_level_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 m
 {
     auto fn = k_count_level<S, SL>;
     constexpr int smem = table_smem_bytes<SL>();
-    static cudaError_t attr = set_smem(fn, smem);
-    if (attr) return attr;
-    static const int per_sm = resident_ctas((const void*)fn, 256, smem);
-    const int grid = full_grid(per_sm, 256, n, sms);
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)fn, 256, smem)) return e;
+    const int grid = full_grid(setup.per_sm, 256, n, sms);
     fn<<<grid, 256, smem, st>>>(lv, start, n, cnt, min_rem);
     return cudaGetLastError();
 }
@@ -134,8 +115,8 @@ cudaError_t count_plan_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 mi
 {
     auto fn = k_count_plan<S, SL>;
     constexpr int smem = table_smem_bytes<SL>();
-    static cudaError_t attr = set_smem(fn, smem);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)fn, 256, smem)) return e;
     fn<<<(n + 255) / 256, 256, smem, st>>>(lv, start, n, cnt, min_rem, offs, cap, plan, done, err, ahead);
     return cudaGetLastError();
 }
@@ -155,8 +136,8 @@ cudaError_t step_t(const LevelView& lv, u32 start, u32 n, u32* cnt, u32 min_rem,
     constexpr int Q = QcapFor<SL, 256>::expand;
     using L = BlockSmem<SL, 256, Q>;
     auto fn = k_step<S, SL, Q>;
-    static cudaError_t attr = set_smem(fn, L::bytes);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)fn, 256, L::bytes)) return e;
     fn<<<1, 256, L::bytes, st>>>(lv, start, n, cnt, min_rem, offs, cap, plan, err, ahead, out, ticket);
     return cudaGetLastError();
 }
@@ -175,8 +156,8 @@ template <class SL>
 cudaError_t count_batch(const Pos* in, u32 n, u32* out, cudaStream_t st)
 {
     constexpr int smem = table_smem_bytes<SL>();
-    static cudaError_t attr = set_smem(k_count_batch<SL>, smem);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)k_count_batch<SL>, 128, smem)) return e;
     k_count_batch<SL><<<small_grid(n, 128), 128, smem, st>>>(in, n, out);
     return cudaGetLastError();
 }
@@ -185,8 +166,8 @@ template <class SL>
 cudaError_t gen_moves_batch(const Pos* in, u32 n, u16* out, u32* nout, cudaStream_t st)
 {
     constexpr int smem = table_smem_bytes<SL>();
-    static cudaError_t attr = set_smem(k_gen_moves_batch<SL>, smem);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)k_gen_moves_batch<SL>, 128, smem)) return e;
     k_gen_moves_batch<SL><<<small_grid(n, 128), 128, smem, st>>>(in, n, out, nout);
     return cudaGetLastError();
 }
@@ -195,8 +176,8 @@ template <class SL>
 cudaError_t gen_boards_batch(const Pos* in, u32 n, Pos* out, u32* nout, cudaStream_t st)
 {
     constexpr int smem = table_smem_bytes<SL>();
-    static cudaError_t attr = set_smem(k_gen_boards_batch<SL>, smem);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)k_gen_boards_batch<SL>, 128, smem)) return e;
     k_gen_boards_batch<SL><<<small_grid(n, 128), 128, smem, st>>>(in, n, out, nout);
     return cudaGetLastError();
 }
@@ -218,8 +199,8 @@ cudaError_t playouts(const Pos& start, u64 seed, u32 n, int min_plies, int max_p
                      int depth_hi, Pos* out, unsigned char* depths, u32* err, cudaStream_t st)
 {
     constexpr int smem = table_smem_bytes<SL>();
-    static cudaError_t attr = set_smem(k_playouts<SL>, smem);
-    if (attr) return attr;
+    static KernelSetup setup;
+    if (const cudaError_t e = setup.once((const void*)k_playouts<SL>, 64, smem)) return e;
     k_playouts<SL><<<small_grid(n, 64), 64, smem, st>>>(start, seed, n, min_plies, max_plies, min_moves, depth_lo,
                                                           depth_hi, out, depths, err);
     return cudaGetLastError();

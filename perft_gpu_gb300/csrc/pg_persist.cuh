@@ -358,26 +358,18 @@ __global__ void __launch_bounds__(PERSIST_T, min_blocks<PERSIST_T>()) k_persist(
 }
 
 constexpr int PERSIST_SMEM = std::max(BlockSmem<SlKS, PERSIST_T, PERSIST_Q>::bytes, LeafSmem<SlKS, PERSIST_T, PERSIST_LEAF_Q>::bytes);
-inline cudaError_t persist_setup_impl()
-{
-    static const cudaError_t e = cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, PERSIST_SMEM);
-    return e;
-}
+static KernelSetup g_persist_setup;
+inline cudaError_t persist_setup_impl() { return g_persist_setup.once((const void*)k_persist, PERSIST_T, PERSIST_SMEM); }
 
 // one CTA per free slot of every SM: all resident, as the barriers need
 inline cudaError_t persist_launch_impl(const PersistArgs& a, cudaStream_t st, int num_sms, int* grid)
 {
-    constexpr int smem = PERSIST_SMEM;
-    int per_sm = 0;
-    cudaError_t e = persist_setup_impl();
+    const cudaError_t e = persist_setup_impl();
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, PERSIST_T, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-    *grid = per_sm * num_sms;
+    *grid = g_persist_setup.per_sm * num_sms;
     PersistArgs copy = a;
     void* args[] = {&copy};
-    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(*grid), dim3(PERSIST_T), args, smem, st);
+    return cudaLaunchCooperativeKernel((const void*)k_persist, dim3(*grid), dim3(PERSIST_T), args, PERSIST_SMEM, st);
 }
 
 }  // namespace pg

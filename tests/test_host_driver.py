@@ -1,0 +1,58 @@
+"""What the host driver asks of the CUDA runtime and launches, without a GPU: the
+library runs over a runtime of host memory and empty kernels (cuda_host.cpp), in
+a process of its own.  Counts are all zero there; what is looked at is which
+kernels a call launches, how, and on which device."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+PRELUDE = """
+import ctypes, os
+import numpy as np
+import perft_gpu_gb300 as pg
+host = ctypes.CDLL(os.environ["LD_PRELOAD"])
+host.host_launches.restype = ctypes.c_char_p
+launches = lambda: [l.split() for l in host.host_launches().decode().splitlines()]
+pos = pg.board_from_fen("rnbqkbnr/pppppppp/8/8/8/8/PPPPPPPP/RNBQKBNR w KQkq - 0 1")
+boards = lambda n: np.repeat(pg.boards_array([pos]), n)
+depths = lambda n, d: np.full(n, d, np.uint8)
+"""
+
+
+@pytest.fixture(scope="module")
+def host_run(tmp_path_factory):
+    nvcc = os.environ.get("NVCC") or shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    if not os.path.exists(os.path.join(include, "cuda_runtime_api.h")):
+        include = "/usr/local/cuda/include"
+    lib = str(tmp_path_factory.mktemp("cuda_host") / "libcuda_host.so")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-w", "-shared", "-fPIC", "-I", include, "-o", lib,
+                           os.path.join(ROOT, "tests", "cuda_host.cpp")])
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code], capture_output=True, text=True, timeout=300,
+                           cwd=ROOT, env=dict(os.environ, PYTHONPATH=ROOT, LD_PRELOAD=lib))
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+@pytest.mark.parametrize("options", ["persistent=True", "persistent=True, graph=True", "graph=True", "",
+                                     "use_tt='dedup'", "slider='ks', block_size=512", "slider='byte', block_size=512"])
+def test_kernels_are_set_up_again_on_another_device(host_run, options):
+    """Dynamic shared memory above 48 KB is allowed for each kernel and device:
+    again after the engine has moved to another one."""
+    host_run("""
+for device in (0, 1):
+    pg.init(device=device)
+    for n in (1, 300, 9000):
+        pg.perft_batch(boards(n), depths(n, 3), %s)
+    pg.count_moves_batch(boards(3))
+    pg.generate_moves(pos)
+    pg.shutdown()
+    assert launches()
+""" % options)
