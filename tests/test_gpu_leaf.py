@@ -173,3 +173,16 @@ def test_one_cta_steps_a_small_level(pg, orc, n):
         got = pg.perft_batch(_copies(pg, fen, n), np.full(n, depth, np.uint8), slider="byte")
         assert np.array_equal(got, pg.perft_batch(_copies(pg, fen, n), np.full(n, depth, np.uint8), slider="ks"))
         assert (got == orc.perft(orc.fen(fen), depth)).all()
+
+
+@pytest.mark.parametrize("slider", ["ks", "byte", "hybrid"])
+@pytest.mark.parametrize("block", [128, 256, 512])
+def test_sparse_leaf_at_every_block_size(pg, orc, slider, block):
+    """A level in which most nodes repeat another, not a whole number of CTAs long."""
+    boards = pg.random_playouts(97, 4000, 2, 60)
+    boards = boards[(boards["pawns"] >> np.uint64(63)) == 0]
+    n = (1 << 19) + 777
+    which = (np.arange(n) // 4) % len(boards)
+    got = pg.perft_batch(boards[which], np.full(n, 2, np.uint8), use_tt="dedup", slider=slider, block_size=block)
+    want, _ = orc.perft_batch(boards, np.full(len(boards), 2, np.uint8), os.cpu_count() or 1)
+    assert np.array_equal(got, want[which])

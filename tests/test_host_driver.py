@@ -56,3 +56,16 @@ for device in (0, 1):
     pg.shutdown()
     assert launches()
 """ % options)
+
+
+@pytest.mark.parametrize("options, threads", [("block_size=128", "128"), ("block_size=512", "512"),
+                                              ("slider='byte', block_size=512", "512"), ("block_size=256", "256")])
+@pytest.mark.parametrize("n", [1000, 1 << 19])
+def test_leaf_runs_the_block_size_asked_for(host_run, options, threads, n):
+    """Also on a level large enough for the leaf that collects its live nodes."""
+    host_run("""
+pg.init()
+pg.perft_batch(boards(%d), depths(%d, 2), use_tt='dedup', %s)
+leaves = [l[1] for l in launches() if 'k_leaf' in l[0]]
+assert leaves and set(leaves) == {%r}, leaves
+""" % (n, n, options, threads))
