@@ -167,7 +167,7 @@ struct Engine {
     u64 stage_cap = 0;
     u64* host_scratch = nullptr;   // pinned small scratch
     unsigned char* host_io = nullptr;  // pinned inputs and counts of a small host-array call
-    bool timing = true;            // the call records its launches' times (it returns stats)
+    bool timing = false;           // the call records its launches' times (it returns stats)
     u64* aux = nullptr;            // small device scratch (input checksum)
     PlanOut* persist_plan = nullptr;  // MAX_LEVELS chunk plans of a persistent launch
     PersistCtl* persist_ctl = nullptr;

@@ -352,6 +352,7 @@ int run_wave(Server& S, std::unique_lock<std::mutex>& lk)
                                                                                  S.wave_grp);
     SRV_CUDA(cudaGetLastError());
     lk.unlock();
+    E.timing = false;  // the last call may have asked for stats; nobody reads a wave's
     E.ticket_next = 0;
     cudaMemsetAsync(E.tickets, 0, MAX_TICKETS * sizeof(u32), E.stream);
     cudaMemsetAsync(E.err, 0, sizeof(u32), E.stream);

@@ -69,3 +69,20 @@ pg.perft_batch(boards(%d), depths(%d, 2), use_tt='dedup', %s)
 leaves = [l[1] for l in launches() if 'k_leaf' in l[0]]
 assert leaves and set(leaves) == {%r}, leaves
 """ % (n, n, options, threads))
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("before", ["", "pg.perft_batch(boards(300), depths(300, 2), slider='ks', stats=pg.PgStats())"])
+def test_served_waves_record_no_timing(host_run, before, persistent):
+    """Whatever the call before them asked for: nobody reads a wave's times."""
+    host_run("""
+pg.init(slider='ks')
+%s
+assert bool(host.host_events()) == bool(%r)
+launches()
+server = pg.Server(slider='ks', persistent=%r)
+assert server.wait(server.submit(pos, 2), timeout=60)[0] == 0
+server.stop()
+assert any('k_gather_wave' in l[0] for l in launches())
+assert host.host_events() == 0
+""" % (before, before, persistent))
