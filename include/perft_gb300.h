@@ -98,7 +98,10 @@ typedef struct pg_opts {
     int use_tt;                  /* pg_tt_mode: PG_TT_OFF, PG_TT_ON, PG_TT_DEDUP_ONLY */
     uint64_t tt_bytes;           /* total TT bytes across depths; 0 = from budget */
     int graph;                   /* replay the call's launch sequence from a captured CUDA graph */
-    pg_stats *stats;             /* optional out */
+    pg_stats *stats;             /* optional out; a call that returns stats times its launches and waits
+                                    for each level's size, where a small call without them launches its
+                                    first levels ahead and several steps in one kernel: the launches
+                                    counted are those of the call with stats */
     int persistent;              /* the whole batch as one persistent cooperative launch that walks
                                     the levels and chunks on the device (Kogge-Stone sliders, 256-thread
                                     CTAs, two-ply leaf; no TT): the reference's device-side driver,

@@ -535,9 +535,8 @@ def perft_bb(pos: HexaBitBoardPosition, depth: int) -> int:
 def perftLauncher(pos: HexaBitBoardPosition, depth: int, launchDepth: int = 0, **kw) -> int:
     """launcher.h:1467-1503: prints "GPU Perft d: n,   Time taken: t seconds,
     nps: r" and returns the count (the reference returns nothing)."""
-    stats = PgStats()
     t0 = time.perf_counter()
-    res = perft(pos, depth, stats=stats, **kw)
+    res = perft(pos, depth, **kw)
     dt = time.perf_counter() - t0
     print("\nGPU Perft %d: %d,   Time taken: %g seconds, nps: %d" % (depth, res, dt, int(res / dt) if dt else 0))
     return res

@@ -47,12 +47,12 @@ def main(argv=None) -> int:
     init(hbm_budget_bytes=a.hbm_budget_mib << 20)
     pos = board_from_fen(fen)
     for d in range(min(a.min_depth, a.depth), a.depth + 1):
-        st = PgStats()
+        st = PgStats() if a.stats else None  # a call that returns stats waits at every level
         t0 = time.perf_counter()
         res = perft(pos, d, slider=a.slider, use_tt=a.tt, tt_bytes=a.tt_mib << 20, stats=st)
         dt = time.perf_counter() - t0
         print("GPU Perft %d: %d,   Time taken: %g seconds, nps: %d" % (d, res, dt, int(res / dt) if dt else 0))
-        if a.stats:
+        if st:
             print("  stats: " + ", ".join("%s=%s" % kv for kv in st.as_dict().items()))
         sys.stdout.flush()
     if a.divide and a.depth >= 1:

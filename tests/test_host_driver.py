@@ -86,3 +86,19 @@ server.stop()
 assert any('k_gather_wave' in l[0] for l in launches())
 assert host.host_events() == 0
 """ % (before, before, persistent))
+
+
+@pytest.mark.parametrize("call", ["cli.main([fen, '4'])", "pg.perftLauncher(pos, 3)"])
+def test_timed_counts_take_the_path_of_a_plain_call(host_run, call):
+    """The command line and the launcher time a call; only --stats asks for the
+    counters, which make it wait for every level's size and record events."""
+    host_run("""
+from perft_gpu_gb300 import cli
+fen = 'rnbqkbnr/pppppppp/8/8/8/8/PPPPPPPP/RNBQKBNR w KQkq - 0 1'
+pg.init(slider='ks')
+%s
+assert any('k_step' in l[0] for l in launches())
+assert host.host_events() == 0
+cli.main([fen, '4', '--stats', '--slider', 'ks'])
+assert host.host_events() > 0
+""" % call.replace("'4']", "'4', '--slider', 'ks']"))
