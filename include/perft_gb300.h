@@ -160,8 +160,9 @@ int pg_perft_batch_device(const pg_board *d_pos, const uint8_t *d_depths, uint32
  * allocating call.  Limits: n <= 65536 positions, depths 0..3, and at most
  * 1,048,576 children of the depth-3 positions per call (both sides to move
  * together).  Larger requests return PG_ERR_CAPACITY; every size check is
- * made before the counting kernels, so d_out then holds zeros.  The first
- * call on a device uploads the move tables (about 0.9 MB, into file-scope
+ * made before any position's count is added up (the children of the depth-3
+ * positions are counted for it), so d_out then holds zeros.  The first call
+ * on a device uploads the move tables (about 0.9 MB, into file-scope
  * device arrays of this library); make that first call before any stream
  * capture.  Every call looks up the array's device address again (no
  * allocation), and a call that finds the tables gone after a device reset
