@@ -1359,6 +1359,8 @@ static int op_batch(int op, const pg_board* pos, u32 n, void* out, u32* nout, in
     Pos* d_in = (Pos*)s;
     void* d_out = s + in_bytes;
     u32* d_n = (u32*)(s + in_bytes + out_bytes);
+    PinnedInputs pinned;
+    pinned.in_use = in_place;
     if (in_place) memcpy(d_in, pos, in_bytes);
     else PG_CUDA(cudaMemcpyAsync(d_in, pos, in_bytes, cudaMemcpyHostToDevice, E.stream));
     if (check) PG_TRY(check_roots_device(d_in, nullptr, pos, nullptr, n));
@@ -1368,6 +1370,7 @@ static int op_batch(int op, const pg_board* pos, u32 n, void* out, u32* nout, in
     else PG_CUDA(ops.gen_boards_batch(d_in, n, (Pos*)d_out, d_n, E.stream));
     if (in_place) {
         PG_CUDA(cudaStreamSynchronize(E.stream));
+        pinned.in_use = false;
         memcpy(out, d_out, out_bytes);
         if (nout) memcpy(nout, d_n, nbytes);
         return PG_OK;

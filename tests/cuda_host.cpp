@@ -52,7 +52,8 @@ void* memory(size_t n) { return calloc(n + 256, 1); }
 
 extern "C" {
 
-// the launches since the last question ("name block" a line), the events recorded
+// the launches since the last question ("name block" a line) and the waits for a
+// stream ("wait"), the events recorded; host_error leaves an error for the next check
 const char* host_launches()
 {
     std::lock_guard<std::mutex> lk(mu);
@@ -60,6 +61,7 @@ const char* host_launches()
     launches.clear();
     return dump.c_str();
 }
+void host_error() { last = cudaErrorInvalidValue; }
 int host_events()
 {
     const int n = events;
@@ -139,7 +141,12 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return cud
 cudaError_t cudaMemcpyToSymbol(const void*, const void*, size_t, size_t, cudaMemcpyKind) { return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)memory(8); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free((void*)s); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t)
+{
+    std::lock_guard<std::mutex> lk(mu);
+    launches += "wait\n";
+    return cudaSuccess;
+}
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)memory(8); return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { free((void*)e); return cudaSuccess; }

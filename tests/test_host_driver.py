@@ -102,3 +102,24 @@ assert host.host_events() == 0
 cli.main([fen, '4', '--stats', '--slider', 'ks'])
 assert host.host_events() > 0
 """ % call.replace("'4']", "'4', '--slider', 'ks']"))
+
+
+@pytest.mark.parametrize("call", ["pg.count_moves_batch(boards(3))", "pg.count_moves_batch(boards(4170))",
+                                  "pg.generate_moves(pos)", "pg.generate_boards(pos)", "pg.perft_divide(pos, 3)",
+                                  "pg.perft_batch(boards(3), depths(3, 2), slider='ks')"])
+def test_a_failed_call_waits_for_what_reads_its_inputs(host_run, call):
+    """An error found behind a launch (here one that somebody else's call left)
+    ends the call; its kernel may still run on the pinned inputs and results, which
+    the next call writes."""
+    host_run("""
+pg.init()
+launches()
+host.host_error()
+try:
+    %s
+    raise SystemExit("no error reported")
+except pg.PerftError as e:
+    assert e.status == 4
+done = launches()
+assert any(l != ["wait"] for l in done) and done[-1] == ["wait"], done
+""" % call)
